@@ -47,7 +47,8 @@ TILE_SHAPES = ((10, 1, 1), (10, 2, 1), (9, 4, 1), (11, 1, 1), (11, 2, 1), (12, 1
 # index-pair shapes of qob_op_tune_ex, in its order: (kets per thread, threads, ket sets per warp)
 PAIR_SHAPES = ((2, 256, 1), (4, 256, 1), (2, 128, 1), (4, 128, 1), (2, 256, 4), (4, 128, 4), (2, 128, 8), (4, 128, 8),
                (2, 128, 16), (4, 128, 16))
-NCANDS = 36 + len(TILE_SHAPES) + len(PAIR_SHAPES)
+# and the flip-form kernel, which sizes itself
+NCANDS = 36 + len(TILE_SHAPES) + len(PAIR_SHAPES) + 1
 SEED_H = 3
 ORACLE_BUILD = ("oracle/liboref.so, g++ -O3 -ffp-contract=off: every multiply and add rounded separately, as the "
                 "reference's Julia code computes; portable flags (no -march=native), the same binary that checks "
@@ -402,9 +403,10 @@ def run_own(args, rank, world, local_rank):
         ms = {f"{1 << (k // 9)}x{SHAPES[k % 9]}": times[k] for k in range(36)}
         ms.update({f"T{b}:{tc}x256s{ls}": times[36 + i] for i, (b, tc, ls) in enumerate(TILE_SHAPES)})
         ms.update({f"{tc}x{blk}s{ls}p": times[36 + len(TILE_SHAPES) + i] for i, (tc, blk, ls) in enumerate(PAIR_SHAPES)})
+        ms["flip"] = times[NCANDS - 1]
         return {"kets_per_thread": v & 0x7F, "index_pairs": bool((v >> 7) & 1), "tile_bits": (v >> 8) & 0xFF,
                 "threads_per_block": (v >> 16) & 0x3FF, "ket_sets_per_warp": 1 << ((v >> 26) & 0x7),
-                "persistent": bool(v >> 30), "ms_by_shape": ms}
+                "persistent": bool(v >> 30), "flip": bool((v >> 29) & 1), "ms_by_shape": ms}
 
     def fix(dt, spec):
         """A launch shape given as <kets per thread>x<threads>[s<ket sets per warp>], P for persistent,
@@ -552,6 +554,8 @@ def run_own(args, rank, world, local_rank):
 
 def kernel_name(scalar, t):
     """The gather kernel a tuned shape runs, as the launch list names it."""
+    if t.get("flip"):
+        return f"k_gather_m<{scalar}, real values, real beta> x 128 threads"
     if t.get("tile_bits"):
         return (f"k_gather_t<{scalar}, real values, {t['kets_per_thread']} kets/thread, real beta> x 256 threads, "
                 f"tiles of 2^{t['tile_bits']} indices, {t['ket_sets_per_warp']} ket sets/warp")

@@ -229,14 +229,18 @@ int qob_op_prepare(qob_ctx* ctx, qob_op* op, int side, int dtype, int64_t* info)
 int qob_op_tune(qob_ctx* ctx, qob_op* op, int side, int dtype, int64_t ncols, double* times_ms,
                 int* chosen);
 
-/* qob_op_tune with the length of times_ms given: writes min(times_len, 58)
+/* qob_op_tune with the length of times_ms given: writes min(times_len, 59)
  * times, the 36 of qob_op_tune, the twelve staged-tile shapes
  * (times_ms[36 + i]) and ten index-pair shapes (times_ms[48 + i], compact
  * plans on kets from the left: two consecutive
  * output indices per thread, see qob_op_set_pairs), (vectors per thread,
  * threads, vector sets per warp) = (2,256,1) (4,256,1) (2,128,1) (4,128,1)
  * (2,256,4) (4,128,4) (2,128,8) (4,128,8) (2,128,16) (4,128,16); *chosen has
- * bit 7 set when an index-pair shape won.  The staged tiles: blocks of 256 threads that copy tiles of 2^bits
+ * bit 7 set when an index-pair shape won.  times_ms[58] is the kernel an operator in
+ * the flip form runs without a tuned shape (every merged group flips a fixed set
+ * of index bits of at most two runs of power-of-two subsystems, with one value:
+ * Pauli strings, bonds and ladder products of spin chains, either side and any
+ * strides; it sizes itself); *chosen has bit 29 set when it won.  The staged tiles: blocks of 256 threads that copy tiles of 2^bits
  * consecutive indices of their kets into shared memory, for (bits, vectors per
  * thread, vector sets per warp) = (10,1,1) (10,2,1) (9,4,1) (11,1,1) (11,2,1)
  * (12,1,1) (9,1,4) (8,1,16) (8,2,8) (9,2,4) (10,1,4) (7,2,16); -1 when not

@@ -534,7 +534,7 @@ int qob_op_prepare(qob_ctx* ctx, qob_op* op, int side, int dtype, int64_t* info)
 }
 
 namespace {
-// The autotuner; writes min(times_len, 58) timings.
+// The autotuner; writes min(times_len, 59) timings.
 int tune_impl(qob_ctx* ctx, qob_op* op, int side, int dtype, int64_t ncols, double* times_ms, int times_len,
               int* chosen) {
   return guard(ctx, [&] {
@@ -560,10 +560,11 @@ int tune_impl(qob_ctx* ctx, qob_op* op, int side, int dtype, int64_t ncols, doub
     const int ptc_c[kPairShapes] = {2, 4, 2, 4, 2, 4, 2, 4, 2, 4};
     const int pblk_c[kPairShapes] = {256, 256, 128, 128, 256, 128, 128, 128, 128, 128};
     const int pls_c[kPairShapes] = {1, 1, 1, 1, 4, 4, 8, 8, 16, 16};
-    constexpr int kCands = 4 * kShapes + kTileShapes + kPairShapes;
+    constexpr int kCands = 4 * kShapes + kTileShapes + kPairShapes + 1;  // the last: k_gather_m
     double t[kCands];
     for (double& v : t) v = -1.0;
     int best = 0, best_block = 256, best_split = 1, best_tile = 0, best_pairs = 0;
+    bool best_flip = false;
     if (P.gather && P.kind == Plan::Kind::Sum) {
       GatherPlan& g = *P.gather;
       const size_t esz = elem_size(dtype);
@@ -610,6 +611,10 @@ int tune_impl(qob_ctx* ctx, qob_op* op, int side, int dtype, int64_t ncols, doub
           ls = tls_c[i];
           tb = tbits_c[i];
           if (!tiles_ok || tb > mbits || tc * ls > ncols) continue;
+        } else if (k == kCands - 1) {
+          if (!g.multi) continue;
+          tc = blk = 0;  // no shape of the other kernels: the flip form's own
+          ls = 1;
         } else {
           const int i = k - 4 * kShapes - kTileShapes;
           tc = ptc_c[i];
@@ -658,6 +663,7 @@ int tune_impl(qob_ctx* ctx, qob_op* op, int side, int dtype, int64_t ncols, doub
           best_split = ls;
           best_tile = tb;
           best_pairs = pr;
+          best_flip = k == kCands - 1;
         }
       }
       g.tc = best;
@@ -672,7 +678,9 @@ int tune_impl(qob_ctx* ctx, qob_op* op, int side, int dtype, int64_t ncols, doub
       for (int k = 0; k < kCands && k < times_len; ++k) times_ms[k] = t[k];
     int lg = 0;
     while ((1 << lg) < best_split) ++lg;
-    if (chosen)
+    if (chosen && best_flip)
+      *chosen = 1 | (128 << 16) | (1 << 29);
+    else if (chosen)
       *chosen = best | (best_pairs << 7) | (best_tile << 8) | ((best_block < 0 ? -best_block : best_block) << 16) |
                 (lg << 26) | (best_block < 0 ? (1 << 30) : 0);
   });

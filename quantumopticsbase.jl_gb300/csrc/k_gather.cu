@@ -62,8 +62,8 @@ __global__ void k_build_diag(int64_t m, int ndg, const GGroup* __restrict__ dg,
   }
 }
 
-// Split of the input vectors into double-float quadruples (re hi, re lo, im
-// hi, im lo), element e of vector c at e * es + c * cs in both arrays.  Each
+// Split of the input vectors into double-float quadruples (re hi, im hi, re
+// lo, im lo: pairs as the packed FP32 instructions take them), element e of vector c at e * es + c * cs in both arrays.  Each
 // thread moves kSplitPer elements a block apart, their loads issued together.
 constexpr int kSplitPer = 4;
 __global__ void __launch_bounds__(256) k_ff_split(const double2* __restrict__ x, int64_t n, int64_t ncols,
@@ -90,8 +90,7 @@ __global__ void __launch_bounds__(256) k_ff_split(const double2* __restrict__ x,
 #pragma unroll
   for (int k = 0; k < kSplitPer; ++k)
     if (o[k] >= 0) {
-      const float2 a = gather::ff_split(v[k].x), b = gather::ff_split(v[k].y);
-      out[o[k]] = make_float4(a.x, a.y, b.x, b.y);
+      out[o[k]] = gather::ff_split4(v[k]);
     }
 }
 

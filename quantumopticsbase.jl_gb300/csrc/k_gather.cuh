@@ -97,7 +97,7 @@ struct Cx<DFX> {
 };
 
 // element type of the input vectors as the kernels read them: the data type,
-// or for DF the (re hi, re lo, im hi, im lo) quadruple written by k_ff_split
+// or for DF the (re hi, im hi, re lo, im lo) quadruple written by k_ff_split
 template <typename R>
 struct In {
   using T = typename Cx<R>::T;
@@ -356,25 +356,26 @@ struct AccFF {
     h = s;
   }
   __device__ void zero() { rh = rl = ih = il = 0.f; }
+  // x: (re hi, im hi, re lo, im lo), as k_ff_split writes it
   __device__ void mac(float2 v, float4 x) {
-    madd(rh, rl, v, x.x, x.y);
-    madd(ih, il, v, x.z, x.w);
+    madd(rh, rl, v, x.x, x.z);
+    madd(ih, il, v, x.y, x.w);
   }
   // (i v) x for real v
   __device__ void mac_i(float2 v, float4 x) {
-    madd(rh, rl, ff_neg(v), x.z, x.w);
-    madd(ih, il, v, x.x, x.y);
+    madd(rh, rl, ff_neg(v), x.y, x.w);
+    madd(ih, il, v, x.x, x.z);
   }
   __device__ void mac(float4 v, float4 x) {
     const float2 vr = make_float2(v.x, v.y), vi = make_float2(v.z, v.w);
-    madd(rh, rl, vr, x.x, x.y);
-    madd(rh, rl, ff_neg(vi), x.z, x.w);
-    madd(ih, il, vr, x.z, x.w);
-    madd(ih, il, vi, x.x, x.y);
+    madd(rh, rl, vr, x.x, x.z);
+    madd(rh, rl, ff_neg(vi), x.y, x.w);
+    madd(ih, il, vr, x.y, x.w);
+    madd(ih, il, vi, x.x, x.z);
   }
   __device__ void mac_i(float4 v, float4 x) { mac(make_float4(-v.z, -v.w, v.x, v.y), x); }
   __device__ void set(float2 v, float4 x) {
-    const float2 r = ff_mul(v, make_float2(x.x, x.y)), i = ff_mul(v, make_float2(x.z, x.w));
+    const float2 r = ff_mul(v, make_float2(x.x, x.z)), i = ff_mul(v, make_float2(x.y, x.w));
     rh = r.x;
     rl = r.y;
     ih = i.x;
@@ -405,7 +406,7 @@ struct AccOf<DF> {
 // AccFF fed with ComplexF64 elements, split as they arrive (DFX)
 __device__ __forceinline__ float4 ff_split4(double2 x) {
   const float2 a = ff_split(x.x), b = ff_split(x.y);
-  return make_float4(a.x, a.y, b.x, b.y);
+  return make_float4(a.x, b.x, a.y, b.y);
 }
 struct AccFFX : AccFF {
   __device__ void mac(float2 v, double2 x) { AccFF::mac(v, ff_split4(x)); }
@@ -942,6 +943,7 @@ __global__ void __launch_bounds__(256) k_gather_c(GatherView g, SiteTable st,
 }  // namespace qob
 
 #include "k_tile.cuh"
+#include "k_multi.cuh"
 
 namespace qob {
 namespace gather {
@@ -1083,6 +1085,13 @@ void launch_tile_tc(const GatherView& v, int tc, const void* x, int64_t xcs, voi
   }
 }
 
+constexpr int64_t kFlipMin = 16384;  // elements of a call from which k_gather_m runs
+
+// k_gather_m on this call (k_multi_{f64,f32,df}.cu)
+template <typename R, int VM>
+void launch_multi(const GatherView& v, const void* x, int64_t xes, int64_t xcs, void* y, int64_t yes, int64_t ycs,
+                  int64_t ncols, c128 alpha, c128 beta, cudaStream_t s);
+
 template <typename R, int VM, bool SQUARE, int BMODE>
 void dispatch_layout(const GatherView& v, const SiteTable& st, int tc, const void* x, int64_t xes,
                      int64_t xcs, void* y, int64_t yes, int64_t ycs, int64_t ncols, typename Cx<R>::T a, typename Cx<R>::T b,
@@ -1165,6 +1174,17 @@ void dispatch_beta(const GatherView& v, const SiteTable& st, int tc, const void*
 template <typename R>
 void dispatch(const GatherView& v, const SiteTable& st, int tc, const void* x, int64_t xes, int64_t xcs,
               void* y, int64_t yes, int64_t ycs, int64_t ncols, c128 alpha, c128 beta, cudaStream_t s) {
+  // the flip form's kernel, unless a shape of the others was tuned or set.  A
+  // ket of a few thousand entries is faster with one index per thread (10 spins,
+  // ComplexF64, 4.7 against 5.2 us; 12 spins, double-float, 6.7 against 7.5);
+  // strided vectors gain at every size.
+  if (v.multi && v.automatic && ncols <= INT32_MAX && (v.m * ncols >= kFlipMin || xes != 1 || yes != 1)) {
+    if (v.real_vals)
+      launch_multi<R, kReal>(v, x, xes, xcs, y, yes, ycs, ncols, alpha, beta, s);
+    else
+      launch_multi<R, kPhased>(v, x, xes, xcs, y, yes, ycs, ncols, alpha, beta, s);
+    return;
+  }
   if (v.real_vals) {
     if (v.square)
       dispatch_beta<R, kReal, true>(v, st, tc, x, xes, xcs, y, yes, ycs, ncols, alpha, beta, s);

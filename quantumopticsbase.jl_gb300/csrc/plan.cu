@@ -381,6 +381,78 @@ static std::vector<c128> eval_slots(const GatherHost& H, const std::vector<TermC
 }
 
 
+// The flip form (k_multi.cuh), when every group has it: at most two runs of
+// power-of-two subsystems, one slot per row in real storage, every stored entry's
+// input index = the output index with the group's flip bits changed, and every
+// stored entry made from the same contributions (so that re-evaluated
+// coefficients keep them equal).  Two 16-byte records per group: the groups that
+// touch the bits below the block of
+// indices per thread first, real groups before imaginary ones.
+static void build_flip_records(GatherPlan& gp, const GatherHost& H, const std::vector<GGroup>& descs,
+                               const std::vector<int>& desc_group, bool store_real) {
+  const uint32_t kLow = (uint32_t)flip_block(gp.precision, gp.ff) - 1;
+  gp.multi = false;
+  gp.two_runs = false;
+  if (!H.S.square || !store_real || descs.empty() || (gp.m & kLow) != 0) return;
+  struct Rec {
+    int order;
+    int4 row, flip;
+  };
+  std::vector<Rec> recs;
+  std::vector<size_t> first(H.groups.size() + 1, H.slots.size());
+  for (size_t s = H.slots.size(); s-- > 0;) first[H.slots[s].group] = s;
+  for (size_t k = 0; k < descs.size(); ++k) {
+    const GGroup& d = descs[k];
+    if (!(d.pow2 && d.nblk >= 1 && d.nblk <= 2 && d.width == 1 && d.nrows <= 32)) return;
+    uint32_t flip = 0;
+    int32_t slot = -1;
+    size_t rep = 0;
+    for (size_t s = first[desc_group[k]]; s < H.slots.size() && H.slots[s].group == desc_group[k]; ++s) {
+      if (!H.live[s]) continue;
+      uint32_t base = 0;  // the row's bits at their places
+      for (int b = 0; b < d.nblk; ++b) base |= (((uint32_t)H.slots[s].r / d.lstride[b]) & (d.mod[b] - 1u)) << (d.shifts[b] & 0xffu);
+      const uint32_t f = base ^ (uint32_t)H.slots[s].coloff;
+      if (slot < 0) {
+        flip = f;
+        slot = H.dst_ell[s];
+        rep = s;
+        continue;
+      }
+      const Slot &a = H.slots[s], &r = H.slots[rep];
+      bool same = f == flip && a.count == r.count;
+      for (int64_t q = 0; same && q < a.count; ++q) {
+        const Contribution &u = H.contrib[a.first + q], &v = H.contrib[r.first + q];
+        same = u.term == v.term && u.pv.re == v.pv.re && u.pv.im == v.pv.im;
+      }
+      if (!same) return;
+    }
+    if (slot < 0) return;
+    const bool two = d.nblk == 2;
+    const uint32_t s1 = d.shifts[0] & 0xffu, s2 = two ? d.shifts[1] & 0xffu : 0u, l2 = two ? d.shifts[1] >> 16 : 0u;
+    uint32_t bits = (d.mod[0] - 1u) << s1;
+    if (two) bits |= (d.mod[1] - 1u) << s2;
+    gp.two_runs |= two;
+    recs.push_back({((bits & kLow) ? 0 : 2) + (d.imag ? 1 : 0),
+                    make_int4((int)(s1 | (s2 << 8) | (l2 << 16)),
+                              (int)((d.mod[0] - 1u) | (two ? (d.mod[1] - 1u) << 16 : 0u)), d.ell_off, d.nrows),
+                    make_int4((int)flip, slot, 0, 0)});
+  }
+  std::stable_sort(recs.begin(), recs.end(), [](const Rec& a, const Rec& b) { return a.order < b.order; });
+  int n[4] = {0, 0, 0, 0};
+  std::vector<int4> out;
+  for (auto& r : recs) {
+    n[r.order]++;
+    out.push_back(r.row);
+    out.push_back(r.flip);
+  }
+  if (n[2] > 32 || n[3] > 32) return;  // one 32-bit mask each
+  gp.nlow_re = n[0];
+  gp.nlow = n[0] + n[1];
+  gp.nre = gp.nlow + n[2];
+  upload_vec(gp.mrec, out);
+  gp.multi = true;
+}
+
 // keep: off-diagonal slots stored even where their value is zero (a factor
 // table's union pattern); complex: store complex values even if all are real.
 static void upload_structure(GatherPlan& gp, GatherHost& H, const std::vector<c128>& val_in,
@@ -427,6 +499,7 @@ static void upload_structure(GatherPlan& gp, GatherHost& H, const std::vector<c1
   };
   // per group: live entries ordered by (r, coloff)
   std::vector<GGroup> descs;
+  std::vector<int> desc_group;  // the group of each descriptor
   std::vector<int32_t> rowptr, coloff, pos_slot;
   std::vector<c128> vals;
   struct EllHost {
@@ -478,6 +551,7 @@ static void upload_structure(GatherPlan& gp, GatherHost& H, const std::vector<c1
         }
       }
       descs.push_back(d);
+      desc_group.push_back((int)gi);
     }
     s0 = s1;
   }
@@ -497,6 +571,7 @@ static void upload_structure(GatherPlan& gp, GatherHost& H, const std::vector<c1
     fastg.push_back(make_int4((int)(d.shifts[0] & 0xffu), (int)(d.mod[0] - 1u), d.ell_off, d.imag));
   }
   if (gp.fast) upload_vec(gp.fastg, fastg);
+  build_flip_records(gp, H, descs, desc_group, store_real);
   gp.square = square;
   upload_vec(gp.groups, descs);
   upload_vec(gp.rowptr, rowptr);
@@ -1084,6 +1159,13 @@ GatherView GatherPlan::view() const {
   v.lane_split = lane_split;
   v.tile_bits = tile_bits;
   v.pairs = pairs;
+  v.multi = multi ? 1 : 0;
+  v.nlow = nlow;
+  v.nlow_re = nlow_re;
+  v.nre = nre;
+  v.two_runs = two_runs ? 1 : 0;
+  v.mrec = (const int4*)mrec.p;
+  v.automatic = tc <= 0 ? 1 : 0;
   v.status = status;
   v.pdl = 0;
   return v;

@@ -156,6 +156,9 @@ struct SiteTable {
   uint64_t mdout[kMaxSites];
 };
 
+// consecutive output indices per thread of k_gather_m
+constexpr int flip_block(int precision, bool ff) { return precision == QOB_C64 && !ff ? 4 : 2; }
+
 // Kernel-side view of a gather plan for one scalar type.
 struct GatherView {
   int64_t m;  // output length
@@ -188,6 +191,11 @@ struct GatherView {
   int32_t pairs;       // 1: compact plans on kets use k_gather_j2 (two consecutive indices per thread)
   int32_t pdl;         // 1: launched with programmatic stream serialization (QOB_OPT_PDL)
   unsigned* status;    // the context's device status word (bounded waits that gave up, failed checks)
+  int32_t multi;       // 1: flip-form records in mrec (k_multi.cuh)
+  int32_t nlow_re, nlow, nre;  // ends of the low real, low imaginary, real groups
+  int32_t two_runs;    // 1: some group has two runs
+  const int4* mrec;    // two per group
+  int32_t automatic;   // 1: no launch shape tuned or set: k_gather_m runs the flip form
 };
 
 // A host-side record of how each stored entry is made from the terms, so a
@@ -261,6 +269,10 @@ struct GatherPlan {
   bool all_w1 = true;
   bool fast = false;
   DeviceBuf fastg;
+  bool multi = false;  // flip-form records (k_multi.cuh)
+  int nlow_re = 0, nlow = 0, nre = 0;
+  bool two_runs = false;
+  DeviceBuf mrec;
   int tc = 0;     // vectors per thread chosen by qob_op_tune (0: automatic)
   int block = 0;  // threads per block chosen by qob_op_tune (0: 256; < 0: persistent grid of -block)
   int lane_split = 1;  // vector sets per warp chosen by qob_op_tune
