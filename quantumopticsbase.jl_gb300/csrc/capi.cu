@@ -70,6 +70,22 @@ c128 coefval(const TermCoef& c, const OpNode* root) {
   return cmul(root->factors[c.top], c.inner);
 }
 
+// Whether an m x n dense matrix on ncols columns runs from its digit planes
+// (k_slice.cu, form QOB_C128, QOB_C64 or QOB_C128X) rather than on the FMA kernels.
+// Measured, FMA -> planes, us.  Dense operators, ComplexF64: n = 4096 on 4 / 16 kets
+// 452 -> 111 / 1737 -> 115, 300 on 16 97 -> 33; double-float 170 -> 104 / 656 -> 109,
+// 61 -> 32; ComplexF32: 4096 on 4 / 8 / 16 61 -> 63 / 90 -> 64 / 157 -> 65, 300 on 16
+// 30 -> 22, 512 on 64 28 -> 28.  Mode products (two): ComplexF64 64 x 2 x 70 on 4 / 16 kets 43 -> 58
+// / 147 -> 58; double-float 64 x 2 x 70 on 16 55 -> 55, 199 x 3 x 201 on 1 143 -> 88;
+// ComplexF32 199 x 3 x 201 on 1 / 15 50 -> 52 / 474 -> 160.
+bool slices_pay(int form, int64_t m, int64_t n, int64_t ncols, bool mode) {
+  if (m < kSliceMin || n < kSliceMin || ncols < 2 || ncols >= (int64_t(1) << 30)) return false;
+  const double flops = 8.0 * m * n * ncols;
+  if (mode) return flops >= (form == QOB_C128 ? 5e7 : form == QOB_C128X ? 1.2e8 : 3e8);
+  if (form == QOB_C64) return ncols >= 8 && flops >= 1e7;
+  return flops >= (ncols >= 4 ? 1e7 : 1e8);
+}
+
 int64_t prod_range(const std::vector<int64_t>& v, size_t lo, size_t hi) {
   int64_t p = 1;
   for (size_t i = lo; i < hi; ++i) p *= v[i];
@@ -104,13 +120,24 @@ void apply_plan(Context& ctx, Plan& P, c128 alpha, const void* x, int64_t xes, i
     for (auto& d : P.dense) {
       // partial sums of a split product in slot ws (free here, as for the split input above);
       // a double-float plan splits x into slot ws + 1 first
+      const c128 ad = cmul(alpha, coefval(d.coef, P.root));
+      const int form = P.ff ? QOB_C128X : P.precision;
+      TcColMap xm, ym;
+      xm.st = xcs;
+      ym.st = ycs;
+      if (!(form == QOB_C64 ? ctx.fp32_tensor : ctx.fp64_tensor && !P.ff) && slices_pay(form, d.m, d.n, ncols, false) &&
+          slice_ready(d.sl, form, d.a.p, d.m, d.n, slice_swap(yes, ym, ncols), s)) {
+        launch_slices(d.sl, form, d.a.p, ad, x, xes, xm, b, y, yes, ym, ncols, s, &ctx.ws, ws,
+                      static_cast<unsigned*>(ctx.status.p), ctx.num_sms, ctx.pdl);
+        b = one;
+        continue;
+      }
       const void* xin = x;
       if (P.ff) {
         void* xs = ctx.ws.get(ws + 1, (size_t)((P.n - 1) * xes + (ncols - 1) * xcs + 1) * 16);
         launch_ff_split(x, P.n, ncols, xes, xcs, xs, s);
         xin = xs;
       }
-      const c128 ad = cmul(alpha, coefval(d.coef, P.root));
       if (ctx.fp32_tensor && P.precision == QOB_C64 && !P.ff && d.m >= kDmmaMinK && d.n >= kDmmaMinK) {
         if (!d.tc.ready) tc_dense_build(d.tc, d.a.p, d.m, d.n, s);
         launch_dense_tc(d.tc, ad, xin, xes, xcs, b, y, yes, ycs, ncols, s, &ctx.ws, ws,
@@ -140,7 +167,24 @@ void apply_plan(Context& ctx, Plan& P, c128 alpha, const void* x, int64_t xes, i
         const c128 ak = (k == 0) ? a : one;
         // a double-float plan splits each step's input into slot ws + 2 (the
         // step's temporaries use ws and ws + 1; sub-plans, which use ws + 2, run after)
-        const bool ffs = P.ff && !st.eye;
+        const int form = P.ff ? QOB_C128X : P.precision;
+        const int64_t pcols = s1 * s3 * ncols;  // the product's columns: (before, after, ket) index triples
+        const bool last = k + 1 == nst;
+        const int64_t len = prod_range(next, 0, next.size());
+        const int64_t out_es = last ? yes : 1, out_cs = last ? ycs : len;
+        TcColMap xm, ym;  // the columns of the input and of the output
+        xm.s1 = ym.s1 = s1;
+        xm.s3 = ym.s3 = s3;
+        xm.sa = ses;
+        xm.sb = s1 * st.din * ses;
+        xm.st = scs;
+        ym.sa = out_es;
+        ym.sb = s1 * st.dout * out_es;
+        ym.st = out_cs;
+        const bool slices = !st.eye && !(form == QOB_C64 ? ctx.fp32_tensor : ctx.fp64_tensor && !P.ff) &&
+                            slices_pay(form, st.dout, st.din, pcols, true) &&
+                            slice_ready(st.sl, form, st.a.p, st.dout, st.din, slice_swap(s1 * out_es, ym, pcols), s);
+        const bool ffs = P.ff && !st.eye && !slices;
         const void* sin = src;
         if (ffs) {
           const int64_t len_in = prod_range(cur, 0, cur.size());
@@ -152,31 +196,25 @@ void apply_plan(Context& ctx, Plan& P, c128 alpha, const void* x, int64_t xes, i
         // (before, after, ket) index triples as columns, contracted dimension din
         const bool tc = ctx.fp32_tensor && P.precision == QOB_C64 && !ffs && !st.eye && st.din >= kDmmaMinK &&
                         st.dout >= kDmmaMinK;
-        auto mode_product = [&](c128 bk, void* out, int64_t oes, int64_t ocs) {
-          if (tc) {
+        auto mode_product = [&](c128 bk, void* out) {
+          unsigned* status = static_cast<unsigned*>(ctx.status.p);
+          if (slices) {
+            launch_slices(st.sl, form, st.a.p, ak, sin, s1 * ses, xm, bk, out, s1 * out_es, ym, pcols, s, &ctx.ws, ws + 3,
+                          status, ctx.num_sms, ctx.pdl);
+          } else if (tc) {
             if (!st.tc.ready) tc_dense_build(st.tc, st.a.p, st.dout, st.din, s);
-            TcColMap xm, ym;
-            xm.s1 = ym.s1 = s1;
-            xm.s3 = ym.s3 = s3;
-            xm.sa = ses;
-            xm.sb = s1 * st.din * ses;
-            xm.st = scs;
-            ym.sa = oes;
-            ym.sb = s1 * st.dout * oes;
-            ym.st = ocs;
-            launch_gemm_tc(st.tc, ak, sin, s1 * ses, xm, bk, out, s1 * oes, ym, s1 * s3 * ncols, s, &ctx.ws, ws + 3,
-                           static_cast<unsigned*>(ctx.status.p), ctx.num_sms, ctx.pdl);
+            launch_gemm_tc(st.tc, ak, sin, s1 * ses, xm, bk, out, s1 * out_es, ym, pcols, s, &ctx.ws, ws + 3, status,
+                           ctx.num_sms, ctx.pdl);
           } else {
-            launch_modek(P.precision, st.a.p, st.eye, s1, st.dout, st.din, s3, ak, sin, ses, scs, bk, out, oes, ocs,
-                         ncols, s, ffs, ctx.fp64_tensor);
+            launch_modek(P.precision, st.a.p, st.eye, s1, st.dout, st.din, s3, ak, sin, ses, scs, bk, out, out_es,
+                         out_cs, ncols, s, ffs, ctx.fp64_tensor);
           }
         };
-        if (k + 1 == nst) {
-          mode_product(b, y, yes, ycs);
+        if (last) {
+          mode_product(b, y);
         } else {
-          const int64_t len = prod_range(next, 0, next.size());
           void* t = ctx.ws.get(ws + (k % 2), (size_t)len * ncols * esz);
-          mode_product(zero, t, 1, len);
+          mode_product(zero, t);
           src = t;
           ses = 1;
           scs = len;

@@ -1,0 +1,998 @@
+// k_slice.cu -- dense operators and the mode products of dense LazyTensor factors
+// (mul! on a DenseOperator, src/operators_dense.jl:394-396, and
+// _tp_matmul_first!/_mid!/_last!, src/operators_lazytensor.jl:281-428) as exact
+// integer products on the 5th-generation tensor cores (tcgen05.mma kind::f16,
+// bf16 operands, FP32 accumulators in tensor memory).
+//
+// GB300's FP64 pipe gives 1.2 TFLOP/s, its FP32 pipes 78, its tensor cores 1900 in
+// bf16.  A bf16 number holds every integer up to 256, so each operand is cut into
+// S signed 8-bit digits of a fixed-point number (Ozaki, Ogita, Oishi & Rump 2012,
+// "Error-free transformations of matrix multiplication"): row i of the matrix
+// relative to 2^ea(i), the power of two above its largest component, vector c
+// relative to 2^ex(c), both per chunk of 256 contracted indices.  The product of
+// two digits is an integer of at most 2^14 and a chunk's sum of the pairs (i, j)
+// with i + j = d at most 256 (d + 1) 2^14: exact in an FP32 accumulator for d <= 3,
+// and beyond that rounding in the accumulator is below 2^-56 of the largest
+// term.  The accumulators of the S diagonals d = 0 .. S - 1 are added as 64-bit
+// integers and rounded once.  The digits:
+//   ComplexF64    S = 8: 62 bits below each row's and vector's largest component
+//                 (a component down to 2^-9 of it keeps all its 53 bits);
+//   double-float  S = 7: 54 bits (its components carry 48);
+//   ComplexF32    S = 4: 30 bits (down to 2^-6 all 24).
+// A vector tile (or matrix) with a component that is not finite, with exponents
+// far from 1 or with a nonzero component below 2^-kGrade of the largest is left to
+// the FMA arithmetic of the form: the split kernel flags the tile, the GEMM does
+// not store it and k_slice_fallback computes it.
+//
+// Layout.  The complex product is one real GEMM as in k_tc32.cu: rows 2i, 2i + 1 of
+// a 128-row tile hold Re and Im of matrix row i, rows j and BN/2 + j of a BN-row
+// tile Re and Im of vector j.  One k step (16 contracted indices) of a tile is S
+// digit planes.  The MMA reads a plane of (rows x 16) bf16 as 8-row groups of two
+// 128-byte core matrices, without a swizzle.  The vectors' planes are stored that
+// way; the matrix's, read for every column tile or streamed once from memory,
+// as bytes in the same order (half the traffic: the matrix's own size again), and
+// four warps widen them to bf16 in shared memory.  Since digit planes 0 .. S - 1 - i
+// of the vectors follow one another, digit i of the matrix times all of them is one
+// MMA of N = (S - i) BN columns (two above 256) into the accumulators of the
+// diagonals i .. S - 1.
+//
+// Block: warp 0 issues the copies, warp 1 owns the tensor memory and
+// issues the MMAs, warp 2 does its waiting (an mbarrier wait by the thread that
+// issued MMAs lasts until they are done; the two meet at a named barrier instead),
+// 6 or 8 warps widen digits and 16 or 8 add up the diagonals and write, beside the
+// next unit's MMAs where the tensor memory holds two sets of accumulators.  Units (column tile, row tile, chunk) in equal runs
+// over one block per SM; a run's part of a row tile either covers it (written to y)
+// or goes to a partial product that k_slice_reduce adds in chunk order.  Waits are
+// bounded as in k_tc32.cu.
+// Measured (device time of a call, FMA kernels -> this; one GB300): two mode products
+// with 199 x 199 and 201 x 201 factors on 15 kets, ComplexF64 4786 -> 341 us,
+// double-float 1331 -> 316, ComplexF32 474 -> 160; a 4096 x 4096 operator on 16 kets
+// 1737 -> 115, 656 -> 109, 157 -> 65.  Error against 128-bit products: ComplexF64
+// 1e-16 (FMA 4e-16), double-float 1e-15 (4e-14), ComplexF32 6e-8 (2e-7).  Bound by
+// the tensor pipe's rate on short MMAs (80 to 110 cycles each up to N = 160) with
+// their commits and, on many columns, by adding up the diagonals (about 9000 cycles
+// per unit beside 13 k steps of 1800).  bf16 planes of the matrix in memory instead of
+// bytes: 370 us and 122 us in ComplexF64.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "k_gather.cuh"  // double-float helpers
+#include "launch.cuh"
+#include "qob_internal.h"
+
+namespace qob {
+
+namespace {
+
+constexpr int kSlChunk = 16;      // k steps of 16 in a chunk
+constexpr int kSlRows = 128;      // real matrix rows of a tile
+constexpr int kSlPolls = 1 << 21;
+constexpr unsigned kSlErrTimeout = 1u;
+constexpr int kGrade = 40;        // nonzero components this far (2^-40) below the largest are left to the FMA form
+
+__device__ __forceinline__ uint32_t saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bar_init(uint64_t* b, unsigned n) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(b)), "r"(n) : "memory");
+}
+__device__ __forceinline__ void bar_expect(uint64_t* b, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(saddr(b)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint64_t* b) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(b)) : "memory");
+}
+__device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t parity) {
+  for (int i = 0; i < kSlPolls; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(saddr(b)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if (i > 64) __nanosleep(32);
+  }
+  return false;
+}
+__device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* b) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   saddr(dst)),
+               "l"(src), "r"(bytes), "r"(saddr(b))
+               : "memory");
+}
+// K-major operand without swizzle: core matrices of 8 rows x 16 bytes, the two of
+// a k step 128 bytes apart, 8-row groups 256 bytes apart; descriptor version 1
+__device__ __forceinline__ uint64_t plane_desc(const void* p) {
+  const uint64_t a = (saddr(p) & 0x3FFFFu) >> 4;
+  return a | (uint64_t(128 >> 4) << 16) | (uint64_t(256 >> 4) << 32) | (uint64_t(1) << 46);
+}
+__device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+      "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
+      : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint64_t* b) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(saddr(b))
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[4]) {  // completion: tcgen05.wait::ld
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[2]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr));
+}
+// two signed bytes (sel picks them into the low bytes of the halves) as bf16: the
+// low seven bits on 128.0 less 128.0, or 256.0 where the sign bit is set (0x4300
+// + 0x80 is 256.0), both exact
+__device__ __forceinline__ uint32_t widen2(uint32_t bytes, uint32_t sel) {
+  const uint32_t h = __byte_perm(bytes, 0x43434343u, sel);
+  uint32_t r;
+  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(h & 0xff7fff7fu), "r"(h & 0xff80ff80u));
+  return r;
+}
+
+// Digits per form, element types, and the fixed-point number of a component:
+// |v| < 2^e times 2^kBits, truncated towards zero.
+template <int FORM>  // QOB_C128, QOB_C64, QOB_C128X
+struct Sl;
+template <>
+struct Sl<QOB_C128> {
+  static constexpr int S = 8;
+  using V = double2;  // vectors
+  using M = double2;  // the stored matrix
+  using F = long long;
+};
+template <>
+struct Sl<QOB_C128X> {
+  static constexpr int S = 7;
+  using V = double2;
+  using M = float4;
+  using F = long long;
+};
+template <>
+struct Sl<QOB_C64> {
+  static constexpr int S = 4;
+  using V = float2;
+  using M = float2;
+  using F = int;
+};
+template <int S>
+constexpr int kBits = 8 * S - 2;
+
+// bits of a component's magnitude, its biased exponent, and whether it is finite
+__device__ __forceinline__ uint32_t mag_hi(double v) { return (uint32_t)__double2hiint(v) & 0x7fffffffu; }
+__device__ __forceinline__ uint32_t mag_hi(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ bool is_nonzero(double v) { return (mag_hi(v) | (uint32_t)__double2loint(v)) != 0u; }
+__device__ __forceinline__ bool is_nonzero(float v) { return mag_hi(v) != 0u; }
+// unbiased exponent e with |v| < 2^e from the high word's bits (subnormals count as the smallest normal)
+template <typename T>
+__device__ __forceinline__ int exp_above(uint32_t hi) {
+  return sizeof(T) == 8 ? (int)(hi >> 20) - 1022 : (int)(hi >> 23) - 126;
+}
+// |eA|, |eX| beyond which a product or its scale could leave the type's range
+template <typename T>
+constexpr int kExpMax = sizeof(T) == 8 ? 400 : 50;
+
+template <int S>
+__device__ __forceinline__ long long fixed_point(double v, int e) {
+  const uint32_t hi = mag_hi(v);
+  const int ev = (int)(hi >> 20);
+  const unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | (ev ? 0x100000u : 0u)) << 32) |
+                               (uint32_t)__double2loint(v);  // 53 bits, |v| = m 2^(max(ev, 1) - 1075)
+  const int sh = kBits<S> - 53 - (e - ((ev ? ev : 1) - 1022));  // m 2^sh
+  long long f = sh >= 0 ? (long long)(m << sh) : sh > -64 ? (long long)(m >> -sh) : 0;
+  return __double2hiint(v) < 0 ? -f : f;
+}
+template <int S>
+__device__ __forceinline__ int fixed_point(float v, int e) {
+  const uint32_t hi = mag_hi(v);
+  const int ev = (int)(hi >> 23);
+  const uint32_t m = (hi & 0x7fffffu) | (ev ? 0x800000u : 0u);
+  const int sh = kBits<S> - 24 - (e - ((ev ? ev : 1) - 126));
+  const int f = sh >= 0 ? (int)(m << sh) : sh > -32 ? (int)(m >> -sh) : 0;
+  return __float_as_int(v) < 0 ? -f : f;
+}
+// the lowest signed digit taken off f
+__device__ __forceinline__ int take_digit(long long& f) {
+  const int d = (int)(signed char)(int)f;
+  f = (f - d) >> 8;
+  return d;
+}
+__device__ __forceinline__ int take_digit(int& f) {
+  const int d = (int)(signed char)f;
+  f = (f - d) >> 8;
+  return d;
+}
+// small integer -> float bits: the mantissa of 1.5 2^23 + d
+__device__ __forceinline__ uint32_t small_float(int d) {
+  return __float_as_uint(__int_as_float(0x4b400000 + d) - 12582912.f);
+}
+
+__device__ __forceinline__ double2 as_value(double2 v) { return v; }
+__device__ __forceinline__ float2 as_value(float2 v) { return v; }
+__device__ __forceinline__ double2 as_value(float4 v) {  // (re hi, re lo, im hi, im lo)
+  return make_double2((double)v.x + (double)v.y, (double)v.z + (double)v.w);
+}
+
+__device__ __forceinline__ int64_t col_offset(const TcColMap& m, int64_t c) {
+  if (m.s1 == 1 && m.s3 == 1) return c * m.st;
+  const uint32_t cc = (uint32_t)c, s1 = (uint32_t)m.s1, s3 = (uint32_t)m.s3;
+  const uint32_t a = cc % s1, q = cc / s1;
+  return (int64_t)a * m.sa + (int64_t)(q % s3) * m.sb + (int64_t)(q / s3) * m.st;
+}
+
+// Digit planes of one tile's chunk: ROWS / 2 vectors (columns of x, or rows of the
+// matrix with INTER) x up to 256 contracted indices.  blockIdx.x: tile, blockIdx.y:
+// chunk.  exps[(tile nch + chunk) ROWS / 2 + vector]: the power of two above its
+// largest component; flags[tile nch + chunk]: 1 where the tile is left to the FMA
+// form (its planes are zero then).  KFAST: threads read along the contracted index.
+constexpr int split_threads(int rows) { return rows == 32 ? 512 : 1024; }
+template <int FORM, int ROWS, bool INTER, typename IN>
+__global__ void __launch_bounds__(split_threads(ROWS)) k_slice_split(const IN* __restrict__ x, int64_t n, int64_t es, TcColMap map,
+                                                     int64_t nvec, int nkb, int kfast, int sub,
+                                                     unsigned char* __restrict__ out,
+                                                     int* __restrict__ exps, int* __restrict__ flags) {
+  constexpr int S = Sl<FORM>::S, H = ROWS / 2, kSlSplit = split_threads(ROWS);
+  using C2 = decltype(as_value(IN{}));
+  using T = decltype(C2{}.x);
+  extern __shared__ __align__(16) unsigned char sl_smem[];
+  __shared__ int ex[H];
+  __shared__ int bad;
+  __shared__ int64_t off[H];
+  pdl_enter();
+  const int kb0 = blockIdx.y * kSlChunk, nks = min(kSlChunk, nkb - kb0);
+  const int64_t k0 = (int64_t)kb0 * 16;
+  const int pitch = sub * 16 + 1;  // sub k steps are staged at a time
+  C2* t = reinterpret_cast<C2*>(sl_smem);  // [vector][k]
+  const int64_t v0 = (int64_t)blockIdx.x * H;
+  if (threadIdx.x == 0) bad = 0;
+  if (threadIdx.x < H) off[threadIdx.x] = v0 + threadIdx.x < nvec ? col_offset(map, v0 + threadIdx.x) : -1;
+  auto stage = [&](int b0) {  // k steps b0 .. of the chunk
+    const int nk = min(sub, nks - b0) * 16;
+    __syncthreads();
+    for (int i = threadIdx.x; i < H * nk; i += kSlSplit) {
+      int v, k;
+      if (kfast) {
+        v = i / nk;
+        k = i - v * nk;
+      } else {
+        k = i / H;
+        v = i - k * H;
+      }
+      const int64_t kg = k0 + b0 * 16 + k;
+      C2 val;
+      val.x = val.y = 0;
+      if (off[v] >= 0 && kg < n) val = as_value(x[off[v] + kg * es]);
+      t[v * pitch + k] = val;
+    }
+    __syncthreads();
+    return nk;
+  };
+  // largest component of each vector, a few threads per vector
+  constexpr int PER = kSlSplit / H;
+  static_assert(PER * H == kSlSplit && PER <= 32, "threads of a vector in one warp");
+  {
+    const int v = threadIdx.x / PER, part = threadIdx.x % PER;
+    uint32_t mx = 0u, mn = 0xffffffffu;
+    for (int b0 = 0; b0 < nks; b0 += sub) {
+      const int nk = stage(b0);
+      for (int k = part; k < nk; k += PER) {
+        const C2 c = t[v * pitch + k];
+        mx = max(mx, max(mag_hi(c.x), mag_hi(c.y)));
+        if (is_nonzero(c.x)) mn = min(mn, mag_hi(c.x));
+        if (is_nonzero(c.y)) mn = min(mn, mag_hi(c.y));
+      }
+    }
+#pragma unroll
+    for (int w = PER / 2; w > 0; w >>= 1) {
+      mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, w));
+      mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, w));
+    }
+    if (part == 0) {
+      const bool any = mn != 0xffffffffu;
+      const int e = any ? exp_above<T>(mx) : 0;
+      ex[v] = e;
+      if (any && (e > kExpMax<T> || e < -kExpMax<T> || e - exp_above<T>(mn) > kGrade)) atomicExch(&bad, 1);
+    }
+  }
+  __syncthreads();
+  const bool skip = bad != 0;
+  const int64_t tile = (int64_t)blockIdx.x * gridDim.y + blockIdx.y;
+  if (threadIdx.x < H) exps[tile * H + threadIdx.x] = ex[threadIdx.x];
+  if (threadIdx.x == 0) flags[tile] = skip ? 1 : 0;
+  for (int b0 = 0; b0 < nks; b0 += sub) {
+    const int nk = sub < nks ? stage(b0) : nks * 16;  // staged already when it is all of the chunk
+    // 8 contracted indices of one real row per task: a store of 16 (INTER: 8) bytes per plane
+    constexpr int kRow = INTER ? 16 : 32;  // bytes of a row in a plane
+    unsigned char* o = out + ((int64_t)blockIdx.x * nkb + kb0 + b0) * (int64_t)(S * ROWS * kRow);
+    for (int i = threadIdx.x; i < ROWS * nk / 8; i += kSlSplit) {
+      const int r = i % ROWS, kc = i / ROWS;  // real row, run of 8 indices
+      const int v = INTER ? r >> 1 : r % H;
+      const bool im = INTER ? (r & 1) : r >= H;
+      uint32_t w[S][INTER ? 2 : 4];
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        const C2 a = t[v * pitch + kc * 8 + 2 * p], b = t[v * pitch + kc * 8 + 2 * p + 1];
+        auto fa = fixed_point<S>(im ? a.y : a.x, ex[v]), fb = fixed_point<S>(im ? b.y : b.x, ex[v]);
+        if (skip) fa = fb = 0;
+#pragma unroll
+        for (int s = S - 1; s >= 0; --s) {
+          const int da = take_digit(fa), db = take_digit(fb);
+          if constexpr (INTER) {
+            const uint32_t two = ((uint32_t)da & 0xffu) | (((uint32_t)db & 0xffu) << 8);
+            w[s][p >> 1] = (p & 1) ? w[s][p >> 1] | (two << 16) : two;
+          } else {
+            w[s][p] = __byte_perm(small_float(da), small_float(db), 0x7632);  // bf16: the upper half of a float
+          }
+        }
+      }
+      unsigned char* q = o + (int64_t)(kc >> 1) * (S * ROWS * kRow) + (r >> 3) * (8 * kRow) + (kc & 1) * (4 * kRow) +
+                         (r & 7) * (kRow / 2);
+#pragma unroll
+      for (int s = 0; s < S; ++s) {
+        if constexpr (INTER)
+          *reinterpret_cast<uint2*>(q + s * (ROWS * kRow)) = make_uint2(w[s][0], w[s][1]);
+        else
+          *reinterpret_cast<uint4*>(q + s * (ROWS * kRow)) = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+      }
+    }
+  }
+}
+
+template <int FORM, int BN>
+struct SlCfg {
+  static constexpr int S = Sl<FORM>::S;
+  static constexpr int kCols = S * BN;                       // columns of one set of accumulators
+  static constexpr int kSets = 2 * kCols <= 512 ? 2 : 1;     // sets in the tensor memory
+  // k steps of a widened buffer (one rendezvous and its commits, ~300 cycles, beside
+  // 80 or more per MMA) and of a stage
+  static constexpr int kG = S == 4 ? 2 : 1, kKs = 2;
+  static constexpr int kA = S * kSlRows * 16, kB = S * BN * 32;  // one k step: bytes of the M side, planes of the N side
+  static constexpr int kWideStep = S * kSlRows * 32;             // one k step of the M side, widened
+  static constexpr int kWide = kG * kWideStep;
+  static constexpr int kWides = BN == 32 ? 2 : 3;
+  static constexpr int kStageA = kKs * kA, kStageB = kKs * kB;
+  static constexpr int kWidenWarps = BN == 32 ? 8 : 6, kAddWarps = BN == 32 ? 8 : 16;
+  static constexpr int kWiden = 32 * kWidenWarps, kWork = 32 * kAddWarps;
+  static constexpr int kThreads = 96 + kWiden + kWork;
+  static constexpr int kBars = 512;
+  // the M side's ring is released as soon as it is widened, the N side's by the MMAs
+  static constexpr int kRingB = BN == 32 ? 3 : 2;
+  static constexpr int kRingA = (226 * 1024 - kBars - kWides * kWide - kRingB * kStageB) / kStageA < 8
+                                    ? (226 * 1024 - kBars - kWides * kWide - kRingB * kStageB) / kStageA
+                                    : 8;
+  static constexpr size_t smem =
+      128 + (size_t)kWides * kWide + (size_t)kRingA * kStageA + (size_t)kRingB * kStageB + kBars;
+  static_assert(kRingA >= 2, "two stages at least");
+  static_assert(8 * (2 * kRingA + 2 * kRingB + 2 * kWides + 2 * kSets + 1) + 8 <= kBars, "barrier area");
+  static_assert(smem <= 227 * 1024, "shared memory of a block");
+};
+
+// H 2^(8 (S - 4)) + L: the sum of the diagonals in units of the last one's
+struct Sum2 {
+  long long h, l;
+};
+template <int S>
+__device__ __forceinline__ Sum2 add_diagonals(const uint32_t (&d)[S]) {
+  auto in = [&](int i) { return (long long)__float2int_rn(__uint_as_float(d[i])); };
+  Sum2 r;
+  r.h = in(0) * (1 << 24) + in(1) * (1 << 16) + in(2) * (1 << 8) + in(3);
+  r.l = 0;
+  if constexpr (S == 8) r.l = in(4) * (1 << 24) + in(5) * (1 << 16) + in(6) * (1 << 8) + in(7);
+  if constexpr (S == 7) r.l = in(4) * (1 << 16) + in(5) * (1 << 8) + in(6);
+  return r;
+}
+// the sum in units of 2^(e - 36 - 8 (S - 4)), rounded to nearest, without the FP64 pipe
+template <int S>
+__device__ __forceinline__ double sum_to_double(Sum2 v, int e) {
+  constexpr int LB = 8 * (S - 4);               // bits of the low part's unit below the high one's
+  long long g = v.h + (v.l >> LB);              // floor
+  unsigned long long f = (unsigned long long)v.l << (64 - LB);  // fraction, in units of 2^-64
+  const bool neg = g < 0;
+  if (neg) {  // -(g + f): complement
+    f = 0ull - f;
+    g = ~g + (f == 0ull ? 1 : 0);
+  }
+  if (g == 0) {  // only a fraction
+    g = (long long)(f >> 32);
+    f <<= 32;
+    e -= 32;
+    if (g == 0) {
+      g = (long long)(f >> 32);
+      f = 0ull;
+      e -= 32;
+      if (g == 0) return 0.0;
+    }
+  }
+  const int s = __clzll(g);  // 1 .. 63
+  unsigned long long m = ((unsigned long long)g << s) | (f >> (64 - s));
+  m = (m >> 11) + ((m >> 10) & 1ull);
+  // value = m 2^(11 - s + e - 36): m has 53 bits
+  const long long bits = ((long long)(1022 + 63 - s + e - 36) << 52) + (long long)m;
+  return __longlong_as_double(bits | (neg ? (long long)0x8000000000000000ull : 0ll));
+}
+
+template <int FORM>
+struct SlAcc {
+  using T = double;
+};
+template <>
+struct SlAcc<QOB_C64> {
+  using T = float;
+};
+
+// part: partial products, [row tile][segment][column][complex row of the tile]
+template <int FORM, int BN>
+__global__ void __launch_bounds__(SlCfg<FORM, BN>::kThreads, 1)
+    k_slice_gemm(const unsigned char* __restrict__ A, const int* __restrict__ ea, const unsigned char* __restrict__ B,
+                 const int* __restrict__ ex, const int* __restrict__ flags, int64_t m, int mt, int64_t ncols, int nkb,
+                 int nch, int per, int64_t units, int smax, int swap, typename Sl<FORM>::V* y, int64_t yes, TcColMap ym,
+                 typename Sl<FORM>::V alpha, typename Sl<FORM>::V beta, typename Sl<FORM>::V* part, unsigned* status) {
+  using C = SlCfg<FORM, BN>;
+  using T = typename SlAcc<FORM>::T;
+  constexpr int S = C::S, NA = C::kRingA, NM = C::kRingB, NW = C::kWides, NB = C::kSets, KS = C::kKs, G = C::kG, H = BN / 2;
+  extern __shared__ __align__(16) unsigned char sl_raw[];
+  unsigned char* base = (unsigned char*)(((uintptr_t)sl_raw + 127) & ~(uintptr_t)127);
+  unsigned char* ring_a = base + (size_t)NW * C::kWide;
+  unsigned char* ring_b = ring_a + (size_t)NA * C::kStageA;
+  uint64_t* afull = reinterpret_cast<uint64_t*>(ring_b + (size_t)NM * C::kStageB);
+  uint64_t* aempty = afull + NA;  // a stage widened (count kWiden)
+  uint64_t* bfull = aempty + NA;
+  uint64_t* bempty = bfull + NM;
+  uint64_t* wfull = bempty + NM;  // a k step of the matrix widened (count kWiden)
+  uint64_t* wempty = wfull + NW;  // and read by its MMAs
+  uint64_t* accf = wempty + NW;   // a unit's accumulators written
+  uint64_t* acce = accf + NB;     // and read (count kWork)
+  uint64_t* fin = acce + NB;      // every MMA issued has completed
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(fin + 1);
+  int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t u0 = (int64_t)blockIdx.x * per;
+  const int nu = (int)(units - u0 < (int64_t)per ? units - u0 : (int64_t)per);
+  const int ch_start = (int)(u0 % nch);
+  auto steps = [&](int ch) { return min(kSlChunk, nkb - ch * kSlChunk); };
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NA; ++s) {
+      bar_init(&afull[s], 1);
+      bar_init(&aempty[s], C::kWiden);
+    }
+    for (int s = 0; s < NM; ++s) {
+      bar_init(&bfull[s], 1);
+      bar_init(&bempty[s], 1);
+    }
+    for (int s = 0; s < NW; ++s) {
+      bar_init(&wfull[s], C::kWiden);
+      bar_init(&wempty[s], 1);
+    }
+    for (int s = 0; s < NB; ++s) {
+      bar_init(&accf[s], 1);
+      bar_init(&acce[s], C::kWork);
+    }
+    bar_init(fin, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(tmem_slot)), "r"(512)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  pdl_enter();
+
+  // warps 1 and 2 meet; true when either asks to stop
+  auto meet = [&](bool ask) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %1, 0;\n\tbar.red.or.pred p, 1, 64, q;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(r)
+        : "r"((uint32_t)ask)
+        : "memory");
+    return r != 0u;
+  };
+  // the roles below walk the same units and k steps: st counts stages, w widened k steps
+  if (warp == 0) {
+    if (lane == 0) {
+      int64_t rt = u0 / nch;
+      int ch = ch_start, st = 0;
+      bool stop = false;
+      for (int u = 0; u < nu && !stop; ++u) {
+        const int64_t mti = rt % mt, ct = rt / mt;
+        const int ks = steps(ch);
+        for (int k = 0; k < ks; k += KS, ++st) {
+          const int sa = st % NA, sb = st % NM;
+          if ((st >= NA && !bar_wait(&aempty[sa], ((st / NA) - 1) & 1)) ||
+              (st >= NM && !bar_wait(&bempty[sb], ((st / NM) - 1) & 1)) || *(volatile int*)abort_flag) {
+            atomicExch(abort_flag, 1);
+            stop = true;
+            break;
+          }
+          const int64_t kb = (int64_t)ch * kSlChunk + k;
+          const uint32_t q = (uint32_t)min(KS, ks - k);
+          bar_expect(&afull[sa], q * C::kA);
+          bulk_copy(ring_a + (size_t)sa * C::kStageA, A + (mti * nkb + kb) * C::kA, q * C::kA, &afull[sa]);
+          bar_expect(&bfull[sb], q * C::kB);
+          bulk_copy(ring_b + (size_t)sb * C::kStageB, B + (ct * nkb + kb) * C::kB, q * C::kB, &bfull[sb]);
+        }
+        if (++ch == nch) {
+          ch = 0;
+          ++rt;
+        }
+      }
+      // every copy issued has landed before the block's shared memory goes away
+      for (int j = max(0, st - NA); j < st; ++j) bar_wait(&afull[j % NA], (j / NA) & 1);
+      for (int j = max(0, st - NM); j < st; ++j) bar_wait(&bfull[j % NM], (j / NM) & 1);
+    }
+  } else if (warp == 1) {
+    // kind::f16: FP32 accumulators, bf16 operands, both K-major, M = 128
+    constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kSlRows >> 4) << 24);
+    int ch = ch_start, st = 0, w = 0;
+    bool stop = false;
+    for (int u = 0; u < nu && !stop; ++u) {
+      const int b = u % NB;
+      const int ks = steps(ch);
+      for (int k0 = 0; k0 < ks; k0 += G, ++w) {
+        const int s = st % NM, c = w % NW, kn = min(G, ks - k0);
+        const bool last = (k0 + G) % KS == 0 || k0 + G >= ks;  // of its stage
+        if (meet(false)) {
+          stop = true;
+          break;
+        }
+        if (lane == 0) {
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint64_t ad0 = plane_desc(base + (size_t)c * C::kWide);
+          const uint64_t bd0 = plane_desc(ring_b + (size_t)s * C::kStageB + (k0 % KS) * C::kB);
+          for (int k = 0; k < kn; ++k) {
+            const uint64_t bd = bd0 + (uint64_t)(k * (C::kB / 16)), ak = ad0 + (uint64_t)(k * (C::kWideStep / 16));
+#pragma unroll
+            for (int i = 0; i < S; ++i) {
+              const uint64_t ad = ak + (uint64_t)(i * (kSlRows * 32 / 16));
+              const uint32_t acc = (i > 0 || k0 + k > 0) ? 1u : 0u;
+#pragma unroll
+              for (int n0 = 0; n0 < (S - i) * BN; n0 += 256) {
+                const int nn = (S - i) * BN - n0 < 256 ? (S - i) * BN - n0 : 256;
+                mma_bf16(tmem + (uint32_t)(b * C::kCols + i * BN + n0), ad, bd + (uint64_t)(n0 * 32 / 16),
+                         kIdesc | ((uint32_t)(nn >> 3) << 17), acc);
+              }
+            }
+          }
+          mma_commit(&wempty[c]);
+          if (last) mma_commit(&bempty[s]);
+          if (k0 + G >= ks) mma_commit(&accf[b]);
+        }
+        __syncwarp();
+        if (last) ++st;
+      }
+      if (++ch == nch) ch = 0;
+    }
+    if (lane == 0) mma_commit(fin);
+  } else if (warp == 2) {
+    int ch = ch_start, st = 0, w = 0;
+    bool stop = false;
+    for (int u = 0; u < nu && !stop; ++u) {
+      const int b = u % NB;
+      const int ks = steps(ch);
+      for (int k0 = 0; k0 < ks && !stop; k0 += G, ++w) {
+        const int s = st % NM, c = w % NW;
+        const bool ok = (k0 > 0 || u < NB || bar_wait(&acce[b], ((u / NB) - 1) & 1)) &&
+                        (k0 % KS != 0 || bar_wait(&bfull[s], (st / NM) & 1)) && bar_wait(&wfull[c], (w / NW) & 1) &&
+                        !*(volatile int*)abort_flag;
+        stop = meet(!__all_sync(0xffffffffu, ok));
+        if ((k0 + G) % KS == 0 || k0 + G >= ks) ++st;
+      }
+      if (++ch == nch) ch = 0;
+    }
+    if (stop) atomicExch(abort_flag, 1);
+  } else if (warp < 3 + C::kWidenWarps) {
+    const int t = threadIdx.x - 96;
+    int ch = ch_start, st = 0, w = 0;
+    bool ok = true;
+    for (int u = 0; u < nu && ok; ++u) {
+      const int ks = steps(ch);
+      for (int k0 = 0; k0 < ks; k0 += G, ++w) {
+        const int s = st % NA, c = w % NW, kn = min(G, ks - k0);
+        if ((k0 % KS == 0 && !bar_wait(&afull[s], (st / NA) & 1)) ||
+            (w >= NW && !bar_wait(&wempty[c], ((w / NW) - 1) & 1)) || *(volatile int*)abort_flag) {
+          atomicExch(abort_flag, 1);
+          ok = false;
+          break;
+        }
+        const uint2* src = reinterpret_cast<const uint2*>(ring_a + (size_t)s * C::kStageA + (k0 % KS) * C::kA);
+        uint4* dst = reinterpret_cast<uint4*>(base + (size_t)c * C::kWide);
+#pragma unroll 4
+        for (int i = t; i < kn * S * kSlRows * 2; i += C::kWiden) {  // 8 digits each
+          const uint2 d = src[i];
+          dst[i] = make_uint4(widen2(d.x, 0x4140), widen2(d.x, 0x4342), widen2(d.y, 0x4140), widen2(d.y, 0x4342));
+        }
+        // the MMAs read through the asynchronous proxy
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        bar_arrive(&wfull[c]);
+        if ((k0 + G) % KS == 0 || k0 + G >= ks) {
+          bar_arrive(&aempty[s]);
+          ++st;
+        }
+      }
+      if (++ch == nch) ch = 0;
+    }
+  } else {
+    // a warp reads the tensor-memory lanes 32 (warp % 4) ..; set h of four warps takes
+    // the vectors [h KQ, (h + 1) KQ): their real columns and, BN/2 on, their imaginary ones
+    const int q4 = warp & 3, half = (warp - 3 - C::kWidenWarps) >> 2;
+    constexpr int KQ = BN / 2 / (C::kAddWarps / 4);
+    constexpr int CG = S == 4 ? 4 : 2;  // columns at a time
+    const uint32_t lane_addr = tmem + ((uint32_t)(q4 * 32) << 16);
+    const int r = q4 * 32 + lane, il = r >> 1;
+    const bool even = (lane & 1) == 0;
+    T acc[KQ];
+#pragma unroll
+    for (int c = 0; c < KQ; ++c) acc[c] = 0;
+    int64_t rt = u0 / nch;
+    int ch = ch_start, ch_first = ch_start;
+    bool ok = true, fresh = true;  // fresh: the segment's first chunk
+    const bool scaled = alpha.x != (T)1 || alpha.y != (T)0, beta_re = beta.x != (T)0, beta_im = beta.y != (T)0;
+    for (int u = 0; u < nu; ++u) {
+      const int b = u % NB;
+      if (!__all_sync(0xffffffffu, bar_wait(&accf[b], (u / NB) & 1) && !*(volatile int*)abort_flag)) {
+        ok = false;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int64_t mti = rt % mt, ct = rt / mt;
+      const int er = ea[(mti * nch + ch) * (kSlRows / 2) + il];
+      // lane c holds the exponent of this warp's vector c
+      const int ec = lane < KQ ? ex[(ct * nch + ch) * H + half * KQ + lane] : 0;
+#pragma unroll 1
+      for (int c0 = 0; c0 < KQ; c0 += CG) {
+        uint32_t p[S][CG], q[S][CG];
+#pragma unroll
+        for (int d = 0; d < S; ++d) {
+          const uint32_t col = lane_addr + (uint32_t)(b * C::kCols + d * BN + half * KQ + c0);
+          tmem_ld(col, p[d]);
+          tmem_ld(col + H, q[d]);
+        }
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        T got[CG];
+#pragma unroll
+        for (int c = 0; c < CG; ++c) {
+          uint32_t dp[S], dq[S];
+#pragma unroll
+          for (int d = 0; d < S; ++d) {
+            dp[d] = p[d][c];
+            dq[d] = q[d][c];
+          }
+          Sum2 a = add_diagonals<S>(dp), o = add_diagonals<S>(dq);
+          // even lane: Re y = Re a Re x - Im a Im x; odd lane: Im y = Im a Re x + Re a Im x
+          o.h = __shfl_xor_sync(0xffffffffu, o.h, 1);
+          a.h += even ? -o.h : o.h;
+          if constexpr (S > 4) {
+            o.l = __shfl_xor_sync(0xffffffffu, o.l, 1);
+            a.l += even ? -o.l : o.l;
+            got[c] = sum_to_double<S>(a, er + __shfl_sync(0xffffffffu, ec, c0 + c));
+          } else {
+            const int e = __shfl_sync(0xffffffffu, ec, c0 + c);
+            got[c] = __ll2float_rn(a.h) * __int_as_float((er - 18 + 127) << 23) * __int_as_float((e - 18 + 127) << 23);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < KQ; j += CG)  // acc[] stays in registers: its index is known
+          if (j == c0) {
+#pragma unroll
+            for (int c = 0; c < CG; ++c) acc[j + c] = fresh ? got[c] : acc[j + c] + got[c];
+          }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      bar_arrive(&acce[b]);
+      const bool closes = ch == nch - 1;
+      if (closes || u == nu - 1) {
+        const bool whole = closes && ch_first == 0;
+        bool skip = false;  // a tile of vectors left to the FMA form
+        for (int j = 0; j < nch; ++j) skip |= flags[(swap ? mti : ct) * nch + j] != 0;
+        const int64_t i = mti * (kSlRows / 2) + il;
+        const int64_t seg = (int64_t)blockIdx.x - (rt * nch) / per;  // segment in the row tile
+        // y offsets: of this lane's M-side row, and in lane c of the warp's N-side row c
+        const int64_t cl = ct * H + half * KQ + lane;
+        const int64_t moff = i >= m ? 0 : swap ? col_offset(ym, i) : i * yes;
+        const int64_t noff = lane >= KQ || cl >= ncols ? 0 : swap ? cl * yes : col_offset(ym, cl);
+        const bool reads = whole && (beta_re || beta_im);
+        T own[KQ];  // y's component of this lane, all loaded before the first is used
+#pragma unroll
+        for (int c = 0; c < KQ; ++c) {
+          own[c] = 0;
+          const int64_t o = moff + __shfl_sync(0xffffffffu, noff, c);
+          if (reads && !skip && i < m && ct * H + half * KQ + c < ncols)
+            own[c] = reinterpret_cast<const T*>(y + o)[lane & 1];
+        }
+#pragma unroll
+        for (int c = 0; c < KQ; ++c) {
+          const T v = acc[c];
+          const bool mine = !skip && i < m && ct * H + half * KQ + c < ncols;
+          const int64_t o = moff + __shfl_sync(0xffffffffu, noff, c);
+          if (!whole) {
+            if (mine)
+              reinterpret_cast<T*>(part + (((rt * smax + seg) * H + half * KQ + c) * (kSlRows / 2) + il))[lane & 1] = v;
+            continue;
+          }
+          // each lane its own component of alpha v + beta y
+          T r = v;
+          if (scaled) {
+            const T w = __shfl_xor_sync(0xffffffffu, v, 1);
+            r = even ? alpha.x * v - alpha.y * w : alpha.x * v + alpha.y * w;
+          }
+          if (beta_im) {
+            const T other = __shfl_xor_sync(0xffffffffu, own[c], 1);
+            r += even ? beta.x * own[c] - beta.y * other : beta.x * own[c] + beta.y * other;
+          } else if (beta_re) {
+            r += beta.x * own[c];
+          }
+          if (mine) reinterpret_cast<T*>(y + o)[lane & 1] = r;
+        }
+        ch_first = 0;
+      }
+      fresh = closes;
+      if (++ch == nch) {
+        ch = 0;
+        ++rt;
+      }
+    }
+    if (!ok) {
+      atomicExch(abort_flag, 1);
+      if (lane == 0 && status) atomicOr(status, kSlErrTimeout);
+    }
+  }
+  if (warp == 1 && lane == 0) bar_wait(fin, 0);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+  }
+}
+
+template <typename V, typename T>
+__device__ __forceinline__ void axpby_out(V* yp, T re, T im, V alpha, V beta) {
+  V o;
+  o.x = alpha.x * re - alpha.y * im;
+  o.y = alpha.x * im + alpha.y * re;
+  if (beta.x != (T)0 || beta.y != (T)0) {
+    const V v = *yp;
+    o.x += beta.x * v.x - beta.y * v.y;
+    o.y += beta.x * v.y + beta.y * v.x;
+  }
+  *yp = o;
+}
+
+// y of the row tiles split over several blocks: their partial products in chunk order
+template <int FORM, int BN>
+__global__ void k_slice_reduce(const typename Sl<FORM>::V* __restrict__ part, const int* __restrict__ flags, int mt,
+                               int nch, int per, int smax, int swap, int64_t m, int64_t ncols,
+                               typename Sl<FORM>::V* y, int64_t yes, TcColMap ym, typename Sl<FORM>::V alpha, typename Sl<FORM>::V beta) {
+  using T = typename SlAcc<FORM>::T;
+  constexpr int H = BN / 2;
+  pdl_enter();
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= m) return;
+  const int il = (int)(i % (kSlRows / 2));
+  const int64_t mti = i / (kSlRows / 2);
+  for (int64_t cg = blockIdx.y; cg < ncols; cg += gridDim.y) {
+    const int64_t ct = cg / H, rt = ct * mt + mti;
+    const int64_t b0 = rt * nch / per, b1 = (rt * nch + nch - 1) / per;
+    if (b0 == b1) continue;  // one block wrote it
+    bool skip = false;
+    for (int j = 0; j < nch; ++j) skip |= flags[(swap ? mti : ct) * nch + j] != 0;
+    if (skip) continue;
+    T re = 0, im = 0;
+    for (int64_t j = 0; j <= b1 - b0; ++j) {
+      const typename Sl<FORM>::V p = part[((rt * smax + j) * H + cg % H) * (kSlRows / 2) + il];
+      re += p.x;
+      im += p.y;
+    }
+    axpby_out(y + (swap ? cg * yes + col_offset(ym, i) : i * yes + col_offset(ym, cg)), re, im, alpha, beta);
+  }
+}
+
+// The flagged column tiles in the form's FMA arithmetic: a thread per row, the
+// tile's vectors one after another.
+template <int FORM>
+__global__ void __launch_bounds__(128) k_slice_fallback(const typename Sl<FORM>::M* __restrict__ a, int64_t m, int64_t n,
+                                                        const typename Sl<FORM>::V* __restrict__ x, int64_t es,
+                                                        TcColMap xm, const int* __restrict__ flags, int nch,
+                                                        int64_t tile, int64_t ncols, typename Sl<FORM>::V* y, int64_t yes,
+                                                        TcColMap ym, typename Sl<FORM>::V alpha,
+                                                        typename Sl<FORM>::V beta) {
+  pdl_enter();
+  const int64_t ct = blockIdx.x;
+  bool run = false;
+  for (int j = 0; j < nch; ++j) run |= flags[ct * nch + j] != 0;
+  if (!run) return;
+  const int64_t i = blockIdx.y * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= m) return;
+  for (int64_t c = ct * tile; c < ncols && c < (ct + 1) * tile; ++c) {
+    const typename Sl<FORM>::V* xc = x + col_offset(xm, c);
+    auto* yp = y + i * yes + col_offset(ym, c);
+    if constexpr (FORM == QOB_C128X) {
+      gather::AccFF acc;
+      acc.zero();
+      for (int64_t k = 0; k < n; ++k) acc.mac(a[i + k * m], gather::ff_split4(xc[k * es]));
+      axpby_out(yp, gather::ff_join(acc.rh, acc.rl), gather::ff_join(acc.ih, acc.il), alpha, beta);
+    } else {
+      using T = typename SlAcc<FORM>::T;
+      T re = 0, im = 0;
+      for (int64_t k = 0; k < n; ++k) {
+        const typename Sl<FORM>::V av = a[i + k * m], xv = xc[k * es];
+        re = fma(av.x, xv.x, re);
+        re = fma(-av.y, xv.y, re);
+        im = fma(av.x, xv.y, im);
+        im = fma(av.y, xv.x, im);
+      }
+      axpby_out(yp, re, im, alpha, beta);
+    }
+  }
+}
+
+template <int FORM, int ROWS, bool INTER, typename IN>
+void run_split(const IN* x, int64_t n, int64_t es, const TcColMap& map, int64_t nvec, int64_t tiles, int nkb,
+               unsigned char* out, int* exps, int* flags, cudaStream_t s, bool pdl) {
+  const int nch = (nkb + kSlChunk - 1) / kSlChunk;
+  auto kern = k_slice_split<FORM, ROWS, INTER, IN>;
+  // k steps staged at a time: the chunk, or half of it where 64 rows of 16 bytes are too many
+  const int sub = ROWS / 2 * sizeof(typename Sl<FORM>::V) <= 512 ? std::min(nkb, kSlChunk) : std::min(nkb, kSlChunk / 2);
+  const size_t smem = (size_t)(ROWS / 2) * (sub * 16 + 1) * sizeof(typename Sl<FORM>::V);
+  QOB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  launch_kernel(pdl, kern, dim3((unsigned)tiles, (unsigned)nch), (unsigned)split_threads(ROWS), smem, s, x, n, es, map, nvec, nkb,
+                es == 1 ? 1 : 0, sub, out, exps, flags);
+  QOB_LAUNCHED();
+}
+
+// swap: the vectors are the M side (their bytes widened), the matrix the N side.
+template <int FORM, int BN>
+void run_slices(const SliceDense& d, bool swap, const void* a, const void* xv, int64_t xes, const TcColMap& xm,
+                int64_t ncols, void* yv, int64_t yes, const TcColMap& ym, c128 al, c128 be, Workspace* ws, int slot,
+                cudaStream_t s, unsigned* status, int num_sms, bool pdl) {
+  using C = SlCfg<FORM, BN>;
+  using V = typename Sl<FORM>::V;
+  using T = typename SlAcc<FORM>::T;
+  constexpr int H = BN / 2, HM = kSlRows / 2;
+  const V* x = static_cast<const V*>(xv);
+  V* y = static_cast<V*>(yv);
+  V alpha, beta;
+  alpha.x = (T)al.re;
+  alpha.y = (T)al.im;
+  beta.x = (T)be.re;
+  beta.y = (T)be.im;
+  const int nkb = d.nkb, nch = (nkb + kSlChunk - 1) / kSlChunk;
+  const int64_t mrows = swap ? ncols : d.m, nrows = swap ? d.m : ncols;
+  const int64_t mt = (mrows + HM - 1) / HM, nt = (nrows + H - 1) / H, vt = swap ? mt : nt;
+  const int64_t rtiles = nt * mt, units = rtiles * nch, wave = num_sms;
+  // equal runs over one wave; whole row tiles when those fill it
+  int64_t per = (units + wave - 1) / wave;
+  if (rtiles >= wave) per = (rtiles + wave - 1) / wave * nch;
+  const int64_t blocks = (units + per - 1) / per;
+  const int smax = (int)((nch - 1) / per + 2);
+  const int64_t tile = swap ? HM : H;  // vectors of a tile
+  const size_t bbytes = (size_t)vt * nkb * (swap ? C::kA : C::kB), ebytes = (size_t)vt * nch * (tile + 1) * sizeof(int);
+  unsigned char* w = static_cast<unsigned char*>(ws->get(slot, bbytes + ebytes));
+  int* exps = reinterpret_cast<int*>(w + bbytes);
+  int* flags = exps + vt * nch * tile;
+  V* part = nullptr;
+  if (per % nch != 0) part = static_cast<V*>(ws->get(slot + 1, (size_t)rtiles * smax * H * HM * sizeof(V)));
+  if (swap)
+    run_split<FORM, kSlRows, true, V>(x, d.n, xes, xm, ncols, vt, nkb, w, exps, flags, s, pdl);
+  else
+    run_split<FORM, BN, false, V>(x, d.n, xes, xm, ncols, vt, nkb, w, exps, flags, s, pdl);
+  const SlicePlanes& pl = swap ? d.nside : d.mside;
+  const unsigned char* mp = swap ? w : static_cast<const unsigned char*>(pl.planes.p);
+  const unsigned char* np = swap ? static_cast<const unsigned char*>(pl.planes.p) : w;
+  const int* me = swap ? exps : static_cast<const int*>(pl.exps.p);
+  const int* ne = swap ? static_cast<const int*>(pl.exps.p) : exps;
+  auto kern = k_slice_gemm<FORM, BN>;
+  QOB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem));
+  launch_kernel(pdl, kern, dim3((unsigned)blocks), (unsigned)C::kThreads, C::smem, s, mp, me, np, ne, (const int*)flags,
+                mrows, (int)mt, nrows, nkb, nch, (int)per, units, smax, swap ? 1 : 0, y, yes, ym, alpha, beta, part,
+                status);
+  QOB_LAUNCHED();
+  if (part) {
+    launch_kernel(pdl, k_slice_reduce<FORM, BN>,
+                  dim3((unsigned)((mrows + 127) / 128), (unsigned)std::min<int64_t>(nrows, 65535)), 128u, 0, s,
+                  (const V*)part, (const int*)flags, (int)mt, nch, (int)per, smax, swap ? 1 : 0, mrows, nrows, y, yes,
+                  ym, alpha, beta);
+    QOB_LAUNCHED();
+  }
+  launch_kernel(pdl, k_slice_fallback<FORM>, dim3((unsigned)vt, (unsigned)((d.m + 127) / 128)), 128u, 0, s,
+                static_cast<const typename Sl<FORM>::M*>(a), d.m, d.n, x, xes, xm, (const int*)flags, nch, tile, ncols,
+                y, yes, ym, alpha, beta);
+  QOB_LAUNCHED();
+}
+
+constexpr int kSwapBN = 64;
+
+// The matrix's planes as the M side (rows widened) or, swap, as the N side.
+template <int FORM>
+void build_slices(SliceDense& d, bool swap, const void* a, cudaStream_t s) {
+  constexpr int S = Sl<FORM>::S;
+  SlicePlanes& pl = swap ? d.nside : d.mside;
+  const int nch = (d.nkb + kSlChunk - 1) / kSlChunk;
+  const int64_t half = swap ? kSwapBN / 2 : kSlRows / 2, tiles = (d.m + half - 1) / half;
+  pl.planes.alloc((size_t)tiles * d.nkb * S * (swap ? kSwapBN * 32 : kSlRows * 16));
+  pl.exps.alloc((size_t)tiles * nch * (half + 1) * sizeof(int));
+  int* exps = static_cast<int*>(pl.exps.p);
+  int* flags = exps + tiles * nch * half;
+  TcColMap map;  // "vectors" = matrix rows, one element apart; contracted index = column, m apart
+  map.st = 1;
+  const auto* m = static_cast<const typename Sl<FORM>::M*>(a);
+  if (swap)
+    run_split<FORM, kSwapBN, false, typename Sl<FORM>::M>(m, d.n, d.m, map, d.m, tiles, d.nkb,
+                                                          static_cast<unsigned char*>(pl.planes.p), exps, flags, s, false);
+  else
+    run_split<FORM, kSlRows, true, typename Sl<FORM>::M>(m, d.n, d.m, map, d.m, tiles, d.nkb,
+                                                         static_cast<unsigned char*>(pl.planes.p), exps, flags, s, false);
+  std::vector<int> f((size_t)(tiles * nch));
+  QOB_CUDA(cudaMemcpyAsync(f.data(), flags, f.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
+  QOB_CUDA(cudaStreamSynchronize(s));
+  pl.state = 1;
+  for (int v : f)
+    if (v) pl.state = -1;
+  if (pl.state < 0) {
+    pl.planes = DeviceBuf();
+    pl.exps = DeviceBuf();
+  }
+}
+
+}  // namespace
+
+// Which side the vectors take: the M side, whose rows lie across lanes, when they
+// (and not the matrix's rows) are next to each other in y.
+bool slice_swap(int64_t yes, const TcColMap& ym, int64_t ncols) {
+  const bool vectors_next = ym.s1 > 1 ? ym.sa == 1 : ym.s3 > 1 ? ym.sb == 1 : ym.st == 1;
+  return yes != 1 && vectors_next && ncols >= kSlRows / 2;
+}
+
+bool slice_ready(SliceDense& d, int form, const void* a, int64_t m, int64_t n, bool swap, cudaStream_t s) {
+  SlicePlanes& pl = swap ? d.nside : d.mside;
+  if (pl.state != 0) return pl.state > 0;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  QOB_CUDA(cudaStreamIsCapturing(s, &cs));
+  if (cs != cudaStreamCaptureStatusNone) return false;  // not built inside a capture
+  d.m = m;
+  d.n = n;
+  d.nkb = (int)((n + 15) / 16);
+  try {
+    if (form == QOB_C128)
+      build_slices<QOB_C128>(d, swap, a, s);
+    else if (form == QOB_C128X)
+      build_slices<QOB_C128X>(d, swap, a, s);
+    else
+      build_slices<QOB_C64>(d, swap, a, s);
+  } catch (const Error& e) {
+    if (e.code != QOB_ERR_OOM) throw;
+    pl.planes = DeviceBuf();  // no room for the planes: the FMA kernels
+    pl.exps = DeviceBuf();
+    pl.state = -1;
+  }
+  return pl.state > 0;
+}
+
+void launch_slices(const SliceDense& d, int form, const void* a, c128 alpha, const void* x, int64_t xes,
+                   const TcColMap& xm, c128 beta, void* y, int64_t yes, const TcColMap& ym, int64_t ncols,
+                   cudaStream_t s, Workspace* ws, int slot, unsigned* status, int num_sms, bool pdl) {
+  const bool swap = slice_swap(yes, ym, ncols);
+#define QOB_SL(F, BN) \
+  run_slices<F, BN>(d, swap, a, x, xes, xm, ncols, y, yes, ym, alpha, beta, ws, slot, s, status, num_sms, pdl)
+  if (form == QOB_C128)
+    ncols <= 16 ? QOB_SL(QOB_C128, 32) : QOB_SL(QOB_C128, kSwapBN);
+  else if (form == QOB_C128X)
+    ncols <= 16 ? QOB_SL(QOB_C128X, 32) : QOB_SL(QOB_C128X, kSwapBN);
+  else
+    ncols <= 16 ? QOB_SL(QOB_C64, 32) : QOB_SL(QOB_C64, kSwapBN);
+#undef QOB_SL
+}
+
+}  // namespace qob

@@ -314,12 +314,25 @@ struct TcColMap {
   int64_t s1 = 1, s3 = 1, sa = 0, sb = 0, st = 0;
 };
 
+// The digit planes of a dense matrix (k_slice.cu) as either side of the product:
+// the one that contiguous kets take made with the plan, the other on first use.
+struct SlicePlanes {
+  int state = 0;  // 0: not made, 1: ready, -1: the matrix is left to the FMA kernels
+  DeviceBuf planes, exps;
+};
+struct SliceDense {
+  int64_t m = 0, n = 0;
+  int nkb = 0;  // k steps of 16
+  SlicePlanes mside, nside;
+};
+
 // Dense full-space term (GEMM / GEMV pass) or a mode-k sequence.
 struct DensePass {
   TermCoef coef;
   int64_t m, n;
   DeviceBuf a;  // m x n column-major in the plan's precision (already transposed for RIGHT)
   TcDense tc;   // ComplexF32 plans: the tensor-core form (QOB_OPT_FP32_TENSOR)
+  SliceDense sl;
 };
 
 
@@ -329,6 +342,7 @@ struct ModekStep {
   DeviceBuf a;  // dout x din column-major
   bool eye = false;
   TcDense tc;   // ComplexF32 plans: the tensor-core form (QOB_OPT_FP32_TENSOR)
+  SliceDense sl;
 };
 struct ModekPass {
   TermCoef coef;
@@ -481,6 +495,17 @@ bool launch_dense_tc(const TcDense& d, c128 alpha, const void* x, int64_t xes, i
 bool launch_gemm_tc(const TcDense& d, c128 alpha, const void* x, int64_t xes, const TcColMap& xm, c128 beta,
                     void* y, int64_t yes, const TcColMap& ym, int64_t ncols, cudaStream_t s, Workspace* ws, int slot,
                     unsigned* status, int num_sms, bool pdl = false);
+// The product of a dense matrix (a: as the FMA kernels read it, form QOB_C128,
+// QOB_C64 or QOB_C128X) from its digit planes (k_slice.cu): columns as
+// launch_gemm_tc's; x unsplit.  slice_swap: which side the vectors take; slice_ready
+// makes the matrix's planes for it if they are not there yet (not inside a capture)
+// and says whether they can be used.  Workspace slots slot, slot + 1.
+constexpr int64_t kSliceMin = 32;  // rows and columns from which a matrix gets planes
+bool slice_swap(int64_t yes, const TcColMap& ym, int64_t ncols);
+bool slice_ready(SliceDense& d, int form, const void* a, int64_t m, int64_t n, bool swap, cudaStream_t s);
+void launch_slices(const SliceDense& d, int form, const void* a, c128 alpha, const void* x, int64_t xes,
+                   const TcColMap& xm, c128 beta, void* y, int64_t yes, const TcColMap& ym, int64_t ncols,
+                   cudaStream_t s, Workspace* ws, int slot, unsigned* status, int num_sms, bool pdl);
 // contracted dimension and kets from which the FP64 tensor-core option
 // applies (an 8 x 8 x 4 tile covers 8 kets: on one ket the FMA kernels are
 // about 15x faster at n = 4096)
