@@ -23,48 +23,11 @@
 
 #include "batch.h"
 #include "k_gather.cuh"
+#include "rk4_stage.cuh"
 
 namespace qob {
 
 namespace {
-
-// k of an RK4 stage into the stage combination (the arithmetic of
-// k_rk4_stage, element by element): 1: acc = k, tmp = psi + dt/2 k; 2, 3:
-// acc += 2 k, tmp = psi + (dt/2 | dt) k; 4: psi += dt/6 (acc + k)
-template <typename CT, typename S>
-__device__ __forceinline__ void rk4_stage_element(const BatchItemDev& it, int64_t j, CT kv, int stage) {
-  CT* psi = (CT*)it.psi;
-  CT* acc = (CT*)it.acc;
-  CT* tmp = (CT*)it.tmp_out;
-  const S dt = (S)it.dt;
-  if (stage == 1) {
-    const CT p = psi[j];
-    const S c = dt * (S)0.5;
-    acc[j] = kv;
-    CT o;
-    o.x = p.x + c * kv.x;
-    o.y = p.y + c * kv.y;
-    tmp[j] = o;
-  } else if (stage == 2 || stage == 3) {
-    const CT p = psi[j];
-    const S c = stage == 2 ? dt * (S)0.5 : dt;
-    CT a = acc[j];
-    a.x += (S)2 * kv.x;
-    a.y += (S)2 * kv.y;
-    acc[j] = a;
-    CT o;
-    o.x = p.x + c * kv.x;
-    o.y = p.y + c * kv.y;
-    tmp[j] = o;
-  } else {
-    const CT a = acc[j];
-    CT p = psi[j];
-    const S c = dt / (S)6;
-    p.x += c * (a.x + kv.x);
-    p.y += c * (a.y + kv.y);
-    psi[j] = p;
-  }
-}
 
 // RK4 instantiates the fused-stage epilogue (stage 1..4 at run time); the
 // plain instantiation keeps the y = alpha k + beta y epilogue alone, so the
@@ -94,11 +57,11 @@ __global__ void __launch_bounds__(256) k_gather_batch(const BatchItemDev* __rest
         CT kv;
         if constexpr (std::is_same<R, gather::DFX>::value || sizeof(R) == 8) {
           gather::combine<0>(&kv, acc[0].total(), it.alpha, it.beta);
-          rk4_stage_element<CT, double>(it, J, kv, stage);
+          rk4_stage_element<CT, double>(it.psi, it.acc, it.tmp_out, it.dt, J, kv, stage);
         } else {
           const float2 a = make_float2((float)it.alpha.x, (float)it.alpha.y);
           gather::combine<0>(&kv, acc[0].total(), a, a);
-          rk4_stage_element<CT, float>(it, J, kv, stage);
+          rk4_stage_element<CT, float>(it.psi, it.acc, it.tmp_out, it.dt, J, kv, stage);
         }
       } else {
         CT* yp = (CT*)it.y + J;

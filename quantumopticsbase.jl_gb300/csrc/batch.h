@@ -59,5 +59,11 @@ void build_tables(Context& ctx, BatchTables& T, const std::vector<BatchSpec>& sp
 void launch_tables(Context& ctx, const BatchTables& T, const std::vector<BatchSpec>& specs, cudaStream_t s,
                    int stage = 0);
 bool all_fused(const BatchTables& T);
+// nsteps RK4 steps of one state in one launch (rk4.cu), work: 3 n elements, waits for
+// the stream; false (nothing done) when the plan or the size is not for it.  Above
+// 2^17 elements a stage is bound by its arithmetic and the launches no longer show.
+constexpr int64_t kRk4GridMax = int64_t(1) << 17;
+bool rk4_one_launch(Context& ctx, const Plan& P, void* psi, void* work, int64_t n, double dt, int nsteps,
+                    cudaStream_t s);
 
 }  // namespace qob

@@ -847,10 +847,16 @@ int qob_rk4(qob_ctx* ctx, qob_op* H, int dtype, void* psi, int64_t n, double dt,
     const size_t sz = (size_t)n * (dtype == QOB_C64 ? 8 : 16);
     char* w = static_cast<char*>(ctx->c.ws.get(20, 3 * sz));
     qob::Plan& P = qob::batch_plan(ctx->c, H, dtype);
+    cudaStream_t st = (cudaStream_t)stream;
+    if (!renormalise && nsteps > 1) {
+      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+      QOB_CUDA(cudaStreamIsCapturing(st, &cs));
+      if (cs == cudaStreamCaptureStatusNone && qob::rk4_one_launch(ctx->c, P, psi, w, n, dt, nsteps, st))
+        return QOB_OK;
+    }
     qob::Ensemble E;
     E.renormalise = renormalise != 0;
     qob::ensemble_build(ctx->c, E, {qob::EvolveState{&P, psi, w, w + sz, w + 2 * sz, n, dt}}, dtype);
-    cudaStream_t st = (cudaStream_t)stream;
     // the first step runs directly (it sizes every buffer); the rest replay a
     // CUDA graph of one step on the context's own stream (the call is
     // synchronous, so the caller's stream is drained first)

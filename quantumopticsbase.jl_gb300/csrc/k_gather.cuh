@@ -424,6 +424,11 @@ struct AccOf<DFX> {
 __device__ __forceinline__ double2 ld(const double2* p) { return __ldg(p); }
 __device__ __forceinline__ float2 ld(const float2* p) { return __ldg(p); }
 __device__ __forceinline__ float4 ld(const float4* p) { return __ldg(p); }
+// CG: inputs that other SMs write during the kernel, read from L2
+template <bool CG, typename T>
+__device__ __forceinline__ T ldx(const T* p) {
+  return CG ? __ldcg(p) : ld(p);
+}
 
 // y = alpha * acc + beta * y with the reference's beta semantics:
 // BMODE 0: beta == 0 (y is not read), 2: general complex beta, 3: real beta.
@@ -566,7 +571,7 @@ __device__ __forceinline__ bool group_row(const GGroup& G, const SiteTable& st, 
 
 // acc[t] = (H x)[J] for the nt vectors starting at xb (element stride es,
 // vector stride xcs).
-template <typename R, int VM, bool SQUARE, bool W1, int TC>
+template <typename R, int VM, bool SQUARE, bool W1, int TC, bool CG = false>
 __device__ __forceinline__ void accumulate(const GatherView& g, const SiteTable& st, const GGroup* sg,
                                            const typename Ell<R, VM != kComplex>::T* ell, uint32_t J,
                                            const typename In<R>::T* xb, int64_t es, int64_t xcs, int nt,
@@ -580,7 +585,7 @@ __device__ __forceinline__ void accumulate(const GatherView& g, const SiteTable&
     const CT* xp = xb + (int64_t)J * es;
 #pragma unroll
     for (int t = 0; t < TC; ++t)
-      if (t < nt) acc[t].set(d, ld(xp + t * xcs));
+      if (t < nt) acc[t].set(d, ldx<CG>(xp + t * xcs));
   } else {
 #pragma unroll
     for (int t = 0; t < TC; ++t) acc[t].zero();
@@ -602,11 +607,11 @@ __device__ __forceinline__ void accumulate(const GatherView& g, const SiteTable&
         if (VM == kPhased && f.w != 0) {
 #pragma unroll
           for (int t = 0; t < TC; ++t)
-            if (t < nt) acc[t].mac_i(v, ld(xp + t * xcs));
+            if (t < nt) acc[t].mac_i(v, ldx<CG>(xp + t * xcs));
         } else {
 #pragma unroll
           for (int t = 0; t < TC; ++t)
-            if (t < nt) acc[t].mac(v, ld(xp + t * xcs));
+            if (t < nt) acc[t].mac(v, ldx<CG>(xp + t * xcs));
         }
       }
     }
@@ -628,11 +633,11 @@ __device__ __forceinline__ void accumulate(const GatherView& g, const SiteTable&
         if (VM == kPhased && G.imag != 0) {
 #pragma unroll
           for (int t = 0; t < TC; ++t)
-            if (t < nt) acc[t].mac_i(v, ld(xp + t * xcs));
+            if (t < nt) acc[t].mac_i(v, ldx<CG>(xp + t * xcs));
         } else {
 #pragma unroll
           for (int t = 0; t < TC; ++t)
-            if (t < nt) acc[t].mac(v, ld(xp + t * xcs));
+            if (t < nt) acc[t].mac(v, ldx<CG>(xp + t * xcs));
         }
       }
     }
@@ -657,11 +662,11 @@ __device__ __forceinline__ void accumulate(const GatherView& g, const SiteTable&
           if (im) {
 #pragma unroll
             for (int t = 0; t < TC; ++t)
-              if (t < nt) acc[t].mac_i(v, ld(xp + t * xcs));
+              if (t < nt) acc[t].mac_i(v, ldx<CG>(xp + t * xcs));
           } else {
 #pragma unroll
             for (int t = 0; t < TC; ++t)
-              if (t < nt) acc[t].mac(v, ld(xp + t * xcs));
+              if (t < nt) acc[t].mac(v, ldx<CG>(xp + t * xcs));
           }
         }
       }
@@ -675,11 +680,11 @@ __device__ __forceinline__ void accumulate(const GatherView& g, const SiteTable&
         if (im) {
 #pragma unroll
           for (int t = 0; t < TC; ++t)
-            if (t < nt) acc[t].mac_i(v, ld(xp + t * xcs));
+            if (t < nt) acc[t].mac_i(v, ldx<CG>(xp + t * xcs));
         } else {
 #pragma unroll
           for (int t = 0; t < TC; ++t)
-            if (t < nt) acc[t].mac(v, ld(xp + t * xcs));
+            if (t < nt) acc[t].mac(v, ldx<CG>(xp + t * xcs));
         }
       }
     }

@@ -559,7 +559,9 @@ static void upload_structure(GatherPlan& gp, GatherHost& H, const std::vector<c1
   gp.nentries = (int64_t)coloff.size();
   gp.all_ell = true;
   gp.all_w1 = true;
+  gp.row_max = 0;
   for (auto& d : descs) {
+    gp.row_max += d.width;
     gp.all_ell &= (d.width > 0);
     gp.all_w1 &= (d.width == 1);
   }

@@ -267,6 +267,7 @@ struct GatherPlan {
   int32_t ell_slots = 0;
   bool all_ell = true;
   bool all_w1 = true;
+  int64_t row_max = 0;  // fixed-width slots of a row, over all groups
   bool fast = false;
   DeviceBuf fastg;
   bool multi = false;  // flip-form records (k_multi.cuh)
@@ -429,6 +430,7 @@ struct Context {
   // device status word (one unsigned, zeroed at creation): kernels record
   // bounded waits that gave up and failed debug checks; read by qob_device_status
   DeviceBuf status;
+  DeviceBuf grid_bar;  // the grid barrier's counter (rk4.cu)
   ~Context();
 };
 
