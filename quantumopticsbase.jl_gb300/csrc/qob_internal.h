@@ -361,11 +361,10 @@ struct SubPass {
 // elements); pre / post phases on the side's order; twiddles of the sign.
 struct FftAxis {
   int64_t n = 0, stride = 1;
-  bool pow2 = true;
-  DeviceBuf tw, pre, post;  // plan precision: n/2 (power of two) or n twiddles; n phases each
-  // four-step split n = n1 * n2 for long power-of-two axes (0: none); all n twiddles
-  int64_t n1 = 0, n2 = 0;
-  DeviceBuf tw_full;
+  bool pow2 = true;  // of at least 8: the FFT, otherwise the direct DFT
+  int sign = 1;
+  DeviceBuf tw, pre, post;  // plan precision: n twiddles, n phases each
+  int64_t n1 = 0, n2 = 0;   // four-step split n = n1 * n2 of long power-of-two axes (0: none)
 };
 
 struct Plan {
