@@ -5,6 +5,7 @@
 #include <cstring>
 #include <new>
 
+#include "fft_line.h"
 #include "qob_internal.h"
 
 namespace qob {
@@ -108,6 +109,17 @@ void apply_plan(Context& ctx, Plan& P, c128 alpha, const void* x, int64_t xes, i
       return;
     }
     c128 b = beta;  // the first pass applies beta, the rest accumulate (:194-197)
+    if (P.subs.size() == 1 && P.gather && P.dense.empty() && P.modek.empty()) {
+      // a diagonal beside a transform -- diagonal -- transform product of the same
+      // coefficient: the product's last pass adds it
+      const Plan& Q = *P.subs[0].plan;
+      const c128 c = Q.kind == Plan::Kind::Product ? cmul(coefval(P.subs[0].coef, P.root), Q.pfactor) : zero;
+      if (Q.kind == Plan::Kind::Product && Q.turn == 0 && Q.chain.size() == 3 && c.re == 1.0 && c.im == 0.0 &&
+          gather_is_diagonal(*P.gather) && P.gather->ff == Q.ff &&
+          launch_fft_turn(ctx, Q, x, xes, xcs, FftOut{y, yes, ycs, alpha, beta, P.gather.get(), x, xes, xcs}, ncols, s,
+                          ws + 4))
+        return;
+    }
     if (P.gather) {
       // a double-float gather splits x into slot ws first (free here: x and y
       // of a nested call live in the caller's slots)
@@ -239,12 +251,12 @@ void apply_plan(Context& ctx, Plan& P, c128 alpha, const void* x, int64_t xes, i
     for (size_t a = 0; a < na; ++a) {
       if (a + 1 == na) {
         void* scratch = P.fft[a].n1 > 0 ? ctx.ws.get(ws + 2, (size_t)P.m * ncols * esz) : nullptr;
-        launch_fft_pass(P.precision, P.fft[a], P.m, src, ses, scs, y, yes, ycs, ncols, alpha, beta, true, scratch,
-                        s, P.ff);
+        launch_fft_pass(ctx, P, a, src, ses, scs, FftOut{y, yes, ycs, alpha, beta, nullptr, nullptr, 0, 0}, ncols,
+                        scratch, s);
       } else {
         void* t = ctx.ws.get(ws + (a % 2), (size_t)P.m * ncols * esz);
-        launch_fft_pass(P.precision, P.fft[a], P.m, src, ses, scs, t, 1, P.m, ncols, one, zero, false, nullptr, s,
-                        P.ff);
+        launch_fft_pass(ctx, P, a, src, ses, scs, FftOut{t, 1, P.m, one, zero, nullptr, nullptr, 0, 0}, ncols, nullptr,
+                        s);
         src = t;
         ses = 1;
         scs = P.m;
@@ -265,6 +277,22 @@ void apply_plan(Context& ctx, Plan& P, c128 alpha, const void* x, int64_t xes, i
   const void* src = x;
   int64_t ses = xes, scs = xcs;
   for (size_t i = 0; i < n; ++i) {
+    if ((int)i == P.turn) {
+      // transform, diagonal, transform in one go
+      Plan& Q = *P.chain[i + 2];
+      const bool last = i + 3 == n;
+      const c128 f = i == 0 ? P.pfactor : one;
+      void* t = last ? y : ctx.ws.get(ws + (i % 2), (size_t)Q.m * ncols * esz);
+      const FftOut o{t, last ? yes : 1, last ? ycs : Q.m, last ? cmul(f, alpha) : f, last ? beta : zero, nullptr, nullptr,
+                     0, 0};
+      if (launch_fft_turn(ctx, P, src, ses, scs, o, ncols, s, ws + 2)) {
+        src = t;
+        ses = 1;
+        scs = Q.m;
+        i += 2;
+        continue;
+      }
+    }
     Plan& Q = *P.chain[i];
     if (i + 1 == n) {
       apply_plan(ctx, Q, alpha, src, ses, scs, beta, y, yes, ycs, ncols, s, ws + 2);

@@ -191,6 +191,17 @@ __device__ __forceinline__ bool nz(float4 v) {
   return ((__float_as_uint(v.x) | __float_as_uint(v.y) | __float_as_uint(v.z) | __float_as_uint(v.w)) << 1) != 0u;
 }
 
+// On GB300 an FP64 instruction with three vector-register operands issues at
+// 1.89 lanes a clock, one with a constant or uniform operand, a multiplication or
+// an addition at 1.60 (8 chains a thread, 32 warps per SM): products are taken as
+// fma(a, b, -0.0), the same number, with its operands in vector registers.
+__device__ __forceinline__ double in_register(double v) {
+  int zero;  // zero, but not to the compiler
+  asm volatile("mov.u32 %0, %%laneid;" : "=r"(zero));
+  return __hiloint2double(__double2hiint(v), __double2loint(v) | (zero >> 5));
+}
+__device__ __forceinline__ float in_register(float v) { return v; }
+
 // FP64 accumulator: plain fused multiply-adds.
 struct AccD {
   double re, im;
@@ -470,6 +481,29 @@ __device__ __forceinline__ void combine(float2* yp, float2 a, float2 alpha, floa
 template <int BMODE>
 __device__ __forceinline__ void combine(double2* yp, float4 a, double2 alpha, double2 beta) {
   combine<BMODE>(yp, make_double2(ff_join(a.x, a.y), ff_join(a.z, a.w)), alpha, beta);
+}
+
+// y = alpha * a + beta * y as combine, FP64 products as fma(a, b, -0.0)
+template <int BMODE>
+__device__ __forceinline__ void combine_nz(double2* o, double2 a, double2 alpha, double2 beta, double nzero) {
+  double re = fma(-alpha.y, a.y, fma(alpha.x, a.x, nzero));
+  double im = fma(alpha.y, a.x, fma(alpha.x, a.y, nzero));
+  if (BMODE == 2) {
+    re = fma(beta.x, o->x, fma(-beta.y, o->y, re));
+    im = fma(beta.x, o->y, fma(beta.y, o->x, im));
+  } else if (BMODE == 3) {
+    re = fma(beta.x, o->x, re);
+    im = fma(beta.x, o->y, im);
+  }
+  *o = make_double2(re, im);
+}
+template <int BMODE>
+__device__ __forceinline__ void combine_nz(double2* o, float4 a, double2 alpha, double2 beta, double nzero) {
+  combine_nz<BMODE>(o, make_double2(ff_join(a.x, a.y), ff_join(a.z, a.w)), alpha, beta, nzero);
+}
+template <int BMODE>
+__device__ __forceinline__ void combine_nz(float2* o, float2 a, float2 alpha, float2 beta, double) {
+  combine<BMODE>(o, a, alpha, beta);
 }
 
 // Copy the group descriptors (then, for plans with the compact form, one int4

@@ -93,17 +93,6 @@ __device__ __forceinline__ f2 sub2(f2 a, f2 b) { return fma2(b, kMinus1, a); }
 template <typename R>
 struct Multi;
 
-// On GB300 an FP64 instruction with three vector-register operands issues at
-// 1.89 lanes a clock, one with a constant or uniform operand, a multiplication or
-// an addition at 1.60 (8 chains a thread, 32 warps per SM): products are taken as
-// fma(a, b, -0.0), the same number, with its operands in vector registers.
-__device__ __forceinline__ double in_register(double v) {
-  int zero;  // zero, but not to the compiler
-  asm volatile("mov.u32 %0, %%laneid;" : "=r"(zero));
-  return __hiloint2double(__double2hiint(v), __double2loint(v) | (zero >> 5));
-}
-__device__ __forceinline__ float in_register(float v) { return v; }
-
 template <>
 struct Multi<double> {
   using X = double2;
@@ -319,29 +308,6 @@ template <typename DT>
 __device__ __forceinline__ void ld_diag(const DT* p, DT* d) {
   d[0] = __ldg(p);
   d[1] = __ldg(p + 1);
-}
-
-// y = alpha * a + beta * y as combine, FP64 products as fma(a, b, -0.0)
-template <int BMODE>
-__device__ __forceinline__ void combine_nz(double2* o, double2 a, double2 alpha, double2 beta, double nzero) {
-  double re = fma(-alpha.y, a.y, fma(alpha.x, a.x, nzero));
-  double im = fma(alpha.y, a.x, fma(alpha.x, a.y, nzero));
-  if (BMODE == 2) {
-    re = fma(beta.x, o->x, fma(-beta.y, o->y, re));
-    im = fma(beta.x, o->y, fma(beta.y, o->x, im));
-  } else if (BMODE == 3) {
-    re = fma(beta.x, o->x, re);
-    im = fma(beta.x, o->y, im);
-  }
-  *o = make_double2(re, im);
-}
-template <int BMODE>
-__device__ __forceinline__ void combine_nz(double2* o, float4 a, double2 alpha, double2 beta, double nzero) {
-  combine_nz<BMODE>(o, make_double2(ff_join(a.x, a.y), ff_join(a.z, a.w)), alpha, beta, nzero);
-}
-template <int BMODE>
-__device__ __forceinline__ void combine_nz(float2* o, float2 a, float2 alpha, float2 beta, double) {
-  combine<BMODE>(o, a, alpha, beta);
 }
 
 // y block = alpha * acc + beta * y block

@@ -1009,11 +1009,14 @@ std::unique_ptr<Plan> compile_plan(Context& ctx, const NodeP& op, int side, int 
     P->root = op.get();
     collect_deps(op.get(), P->deps);
     const size_t k = op->ops.size();
+    std::vector<const OpNode*> ops;
     for (size_t i = 0; i < k; ++i) {
       // LEFT applies the last operator first; RIGHT the first
       const NodeP& c = tr ? op->ops[i] : op->ops[k - 1 - i];
       P->chain.push_back(compile_plan(ctx, c, side, precision));
+      ops.push_back(c.get());
     }
+    find_fft_turn(*P, ops);
     P->nterms_total = (int)k;
     return P;
   }

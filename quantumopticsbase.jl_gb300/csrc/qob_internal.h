@@ -382,6 +382,8 @@ struct Plan {
   // Product
   c128 pfactor{1.0, 0.0};
   std::vector<std::unique_ptr<Plan>> chain;  // in application order
+  int turn = -1;  // >= 0: chain[turn] .. chain[turn + 2] are transform, diagonal, transform (fft.cu)
+  DeviceBuf mid;  // the phases between those two, last axis
   // Fft
   std::vector<FftAxis> fft;
   // dependency record: (node, factors_version) of every LazySum inside
@@ -461,9 +463,13 @@ void launch_td_advance(long long* step, cudaStream_t s);
 // (beta ignored when final == false: y is overwritten).
 // scratch (len * ncols elements, may be null) lets few long lines run as a
 // four-step FFT over many blocks.
-void launch_fft_pass(int precision, const FftAxis& ax, int64_t len, const void* x, int64_t xes, int64_t xcs,
-                     void* y, int64_t yes, int64_t ycs, int64_t ncols, c128 alpha, c128 beta, bool final,
-                     void* scratch, cudaStream_t s, bool ff = false);
+struct FftOut;
+void launch_fft_pass(Context& ctx, const Plan& P, size_t a, const void* x, int64_t xes, int64_t xcs, const FftOut& o,
+                     int64_t ncols, void* scratch, cudaStream_t s);
+bool gather_is_diagonal(const GatherPlan& g);
+void find_fft_turn(Plan& P, const std::vector<const OpNode*>& ops);
+bool launch_fft_turn(Context& ctx, const Plan& P, const void* x, int64_t xes, int64_t xcs, const FftOut& o,
+                     int64_t ncols, cudaStream_t s, int ws);
 std::unique_ptr<Plan> compile_fft(const NodeP& op, int side, int precision);
 int gather_tile(const GatherPlan& g, int64_t ncols);
 void launch_scale(int precision, void* y, int64_t rows, int64_t cols, int64_t ld_row,

@@ -27,8 +27,8 @@ def _dev(a, form):
     return torch.as_tensor(np.ascontiguousarray(a.T)).to(torch.complex64 if form == "c64" else torch.complex128).cuda().t()
 
 
-def _check(T, cols, left, seed):
-    """T A (left) or A T on `cols` columns / rows, all scalar forms and precisions."""
+def _check(T, cols, left, seed, scalars=((1.0, 0.0), (AL, 0.0), (1.0, 1.0), (AL, BE))):
+    """T A (left) or A T on `cols` columns / rows, scalar forms and precisions."""
     from qobgpu.mul import mul_
 
     n, g = len(T.basis_l), Q.GenericBasis(cols)
@@ -36,7 +36,7 @@ def _check(T, cols, left, seed):
     shape = (n, cols) if left else (cols, n)
     a, y = (np.asfortranarray(rng.complex_normal(n * cols).reshape(shape, order="F")) for _ in range(2))
     bl, br = ((T.basis_l, g), (T.basis_r, g)) if left else ((g, T.basis_r), (g, T.basis_l))
-    for al, be in ((1.0, 0.0), (AL, 0.0), (1.0, 1.0), (AL, BE)):
+    for al, be in scalars:
         A, Y = O.Operator(*br, a), O.Operator(*bl, y)
         ref = OR.mul(Y, T, A, al, be) if left else OR.mul(Y, A, T, al, be)
         for form, tol in (("c128", 1e-12), ("c64", 1e-5), ("ff", 1e-12)):
@@ -66,3 +66,29 @@ def test_axes(shape):
     bxs = [PositionBasis(-3.0 - i, 4.0 + i, n) for i, n in enumerate(shape)]
     T = transform(Q.tensor_basis(*[MomentumBasis(b) for b in bxs]), Q.tensor_basis(*bxs))
     _check(T, 3, True, 950 + len(shape))
+
+
+def _diag(b, rng, real):
+    v = rng.complex_normal(len(b))
+    return O.Operator(b, b, O.spdiagm(len(b), len(b), {0: v.real.copy() if real else v}))
+
+
+@pytest.mark.parametrize("shape", [(8,), (64,), (512,), (2048,), (8, 16), (3, 32), (32, 3), (16, 8, 32), (16, 512)])
+@pytest.mark.parametrize("cols", [1, 170])
+@pytest.mark.parametrize("left", [True, False])
+def test_transform_diagonal_transform(shape, cols, left):
+    """Products T' D T: alone, in a longer chain, and beside diagonal terms of the same and
+    of other coefficients; lengths with equal and unequal four-step halves, last axes with and
+    without an FFT, lines that only the four-step form spreads."""
+    bxs = [PositionBasis(-3.0 - i, 4.0 + i, n) for i, n in enumerate(shape)]
+    X = bxs[0] if len(bxs) == 1 else Q.tensor_basis(*bxs)
+    cols = min(cols, 2**18 // len(X))  # the oracle's time
+    P = MomentumBasis(X) if len(bxs) == 1 else Q.tensor_basis(*[MomentumBasis(b) for b in bxs])
+    rng = Q.Rng(970 + len(X) + cols)
+    real = cols == 1
+    T, Ti, D, V = transform(P, X), transform(X, P), _diag(P, rng, real), _diag(X, rng, not real)
+    prod = O.LazyProduct((Ti, D, T))
+    _check(prod, cols, left, 1, scalars=((AL, BE),))
+    _check(O.LazyProduct((V, Ti, D, T)), cols, left, 2, scalars=((1.0, 0.0),))
+    for cs in ([1.0, 1.0], [0.5, 2.0 - 1j]):
+        _check(O.LazySum(X, X, cs, (prod, V)), cols, left, 3, scalars=((-1j, 0.0), (AL, BE)))
