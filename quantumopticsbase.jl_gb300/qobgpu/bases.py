@@ -27,7 +27,8 @@ class Basis:
         return (type(self).__name__, self.shape)
 
     def __eq__(self, other) -> bool:
-        return isinstance(other, Basis) and self._key() == other._key()
+        # one object is the usual case on the call path: no keys of every subsystem
+        return self is other or (isinstance(other, Basis) and self._key() == other._key())
 
     def __hash__(self) -> int:
         return hash(self._key())

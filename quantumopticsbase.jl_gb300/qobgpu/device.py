@@ -132,6 +132,7 @@ def _build(ctx: Context, op) -> Handle:
         h = _new(lib.qob_op_lazysum, ctx, len(op.basis_l), len(op.basis_r), len(kids), _c_array(f, C.c_double), arr)
         hd = Handle(ctx, h, kids)
         hd.factors_seen = op.factors.copy()
+        hd.factors_bytes = hd.factors_seen.tobytes()
         return hd
     if isinstance(op, O.LazyProduct):
         kids = [handle(ctx, o) for o in op.operators]
@@ -161,23 +162,38 @@ def handle(ctx: Context, op) -> Handle:
     h = cache.get(ctx.device)
     if h is None:
         h = _build(ctx, op)
+        h.sums = _inner_sums(op, h)
         cache[ctx.device] = h
     else:
-        _sync_factors(ctx, op, h)
+        if isinstance(op, O.LazySum):
+            _sync_factors(ctx, op, h)
+        for s, k in h.sums:
+            _sync_factors(ctx, s, k)
     return h
 
 
+def _inner_sums(op, h: Handle) -> list:
+    """The LazySums inside op whose factors may change, outermost first (not op itself:
+    a handle that held its operator would keep both from being freed)."""
+    out = []
+    if isinstance(op, (O.LazySum, O.LazyProduct)):
+        for o, k in zip(op.operators, h.children):
+            if isinstance(o, O.LazySum):
+                out.append((o, k))
+            out += _inner_sums(o, k)
+    return out
+
+
 def _sync_factors(ctx: Context, op, h: Handle) -> None:
-    if isinstance(op, O.LazySum):
-        if not np.array_equal(h.factors_seen, op.factors):
-            f = np.ascontiguousarray(op.factors, np.complex128).view(np.float64)
-            raise_for(L.lib().qob_op_set_factors(ctx.ptr, h.ptr, _c_array(f, C.c_double)), ctx)
-            h.factors_seen = op.factors.copy()
-        for o, k in zip(op.operators, h.children):
-            _sync_factors(ctx, o, k)
-    elif isinstance(op, (O.LazyProduct,)):
-        for o, k in zip(op.operators, h.children):
-            _sync_factors(ctx, o, k)
+    f = op.factors
+    # the bytes first: an unchanged sum's call pays for no array comparison
+    if type(f) is np.ndarray and f.tobytes() == h.factors_bytes and f.dtype == np.complex128:
+        return
+    if not np.array_equal(h.factors_seen, op.factors):
+        f = np.ascontiguousarray(op.factors, np.complex128).view(np.float64)
+        raise_for(L.lib().qob_op_set_factors(ctx.ptr, h.ptr, _c_array(f, C.c_double)), ctx)
+        h.factors_seen = op.factors.copy()
+    h.factors_bytes = np.asarray(op.factors, np.complex128).tobytes()
 
 
 def prepare(op, side: int = L.QOB_LEFT, dtype=np.complex128, device: int = 0) -> dict:

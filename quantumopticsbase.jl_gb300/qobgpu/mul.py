@@ -24,8 +24,15 @@ from .device import dtype_code, get_context, handle, raise_for
 from .states import Bra, Ket, StateVector
 
 
+_torch_types: dict[type, bool] = {}
+
+
 def _is_torch(a) -> bool:
-    return type(a).__module__.startswith("torch")
+    t = type(a)
+    r = _torch_types.get(t)
+    if r is None:
+        r = _torch_types[t] = t.__module__.startswith("torch")
+    return r
 
 
 def _state_like(o) -> bool:
@@ -41,16 +48,20 @@ def _np_dtype(a):
 
 
 def _stream_ptr(device: int):
+    """The current stream's pointer (asked for without a Stream object where torch has that)."""
     import torch
 
-    return C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw(device) if raw is not None else torch.cuda.current_stream(device).cuda_stream
 
 
 def _matrix_view(a):
     """(rows, cols, ld) of a 1-D or column-major 2-D array/tensor."""
-    if a.ndim == 1:
-        return a.shape[0], 1, max(1, a.shape[0])
-    r, c = a.shape
+    shape = a.shape
+    if len(shape) == 1:
+        r = shape[0]
+        return r, 1, r or 1
+    r, c = shape
     if _is_torch(a):
         st = a.stride()
         if st[0] != 1 and r > 1:
@@ -103,13 +114,15 @@ def mul_(result, a, b, alpha=1.0, beta=0.0, device: int | None = None, arith: st
     if _is_torch(y):
         import torch
 
-        dev = y.device.index if device is None else device
+        where = y.device
+        dev = where.index if device is None else device
         ctx = get_context(dev)
         h = handle(ctx, op)
-        ydt = _np_dtype(y)
-        if not _is_torch(x) or x.device != y.device or _np_dtype(x) != ydt:
-            xt = torch.as_tensor(np.asarray(x) if not _is_torch(x) else x, device=y.device)
-            x = xt.to(torch.complex64 if ydt == np.complex64 else torch.complex128)
+        f32 = y.dtype == torch.complex64
+        # the same dtype: both of them complex64 or, as _np_dtype has it, neither
+        if not _is_torch(x) or x.device != where or (x.dtype == torch.complex64) != f32:
+            xt = torch.as_tensor(np.asarray(x) if not _is_torch(x) else x, device=where)
+            x = xt.to(torch.complex64 if f32 else torch.complex128)
             if x.ndim == 2 and x.stride(0) != 1 and x.shape[0] > 1:
                 x = x.t().contiguous().t()
         xr, xc, xld = _matrix_view(x)
@@ -117,10 +130,11 @@ def mul_(result, a, b, alpha=1.0, beta=0.0, device: int | None = None, arith: st
         if side == L.QOB_RIGHT and x.ndim == 1:
             xr, xc, xld = 1, x.shape[0], 1
             yr, yc, yld = 1, y.shape[0], 1
-        rc = lib.qob_mul(ctx.ptr, side, int(is_vec), h.ptr, _code(ydt, arith), alpha.real, alpha.imag,
-                         C.c_void_p(x.data_ptr()), xr, xc, xld, beta.real, beta.imag, C.c_void_p(y.data_ptr()),
-                         yr, yc, yld, _stream_ptr(dev))
-        raise_for(rc, ctx)
+        code = (L.QOB_C64 if f32 else L.QOB_C128) if arith is None else _code(_np_dtype(y), arith)
+        rc = lib.qob_mul(ctx.ptr, side, is_vec, h.ptr, code, alpha.real, alpha.imag, x.data_ptr(), xr, xc, xld,
+                         beta.real, beta.imag, y.data_ptr(), yr, yc, yld, _stream_ptr(dev))
+        if rc:
+            raise_for(rc, ctx)
         return result
     # host arrays: copy in, apply on the device, copy back
     dev = 0 if device is None else device
