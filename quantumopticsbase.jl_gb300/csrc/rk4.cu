@@ -16,12 +16,14 @@
 // threads, and rows too wide for the list, walk the compiled tables at each stage
 // (k_rk4_grid).
 //
-// What bounds it: the barrier and one round trip to L2 per stage, 3.2 us where the
-// launches took 8.2.  Blocks of 128: 64 need twice the arrivals at the counter, 256
-// leave SMs without a block (100 steps, ComplexF64, us for 64 / 128 / 256: 10 spins 1178 / 1077 /
-// 1293, 12 1271 / 1282 / 1533, 14 1370 / 1327 / 1722, 16 3445 / 2820 / 2750).  Against
-// four launches per step: 8 spins 2666 -> 1010, 12 3294 -> 1282, 14 3697 -> 1327,
-// 16 4552 -> 2801, 17 7608 -> 5130.
+// What bounds it: the barrier, one round trip to L2 and the chain of a row's dependent
+// multiply-adds per stage, 3.1 us where the launches took 8.2.  Blocks of 128: 64 need
+// twice the arrivals at the counter, 256 leave SMs without a block (100 steps,
+// ComplexF64, us for 64 / 128 / 256: 10 spins 1178 / 1077 / 1293, 12 1271 / 1282 /
+// 1533, 14 1370 / 1327 / 1722, 16 3445 / 2820 / 2750).  Against four launches per step
+// (ComplexF64 / ComplexF32 / double-float): 8 spins 2670 -> 776 / 2264 -> 579 / 2675 -> 972,
+// 12 3285 -> 1224 / 2880 -> 926 / 3493 -> 1451, 16 4518 -> 2701 / 3667 -> 1422 / 4516 -> 2385,
+// 17 7608 -> 5071 (ComplexF64).
 //
 // Waits are bounded: a block that gives up marks the counter, every block leaves at
 // its next barrier, the context's status word says so and the call fails.
@@ -47,6 +49,15 @@ struct Rk4Args {
   int nsteps;
   unsigned* bar;
 };
+
+// -i v: a swap and a sign, where products with (0, -1) would be four FP64 operations
+__device__ __forceinline__ double2 minus_i(double2 v) {
+  return make_double2(v.y, __hiloint2double(__double2hiint(v.x) ^ (int)0x80000000, __double2loint(v.x)));
+}
+__device__ __forceinline__ float2 minus_i(float2 v) { return make_float2(v.y, -v.x); }
+__device__ __forceinline__ double2 minus_i(float4 v) {
+  return minus_i(make_double2(gather::ff_join(v.x, v.y), gather::ff_join(v.z, v.w)));
+}
 
 // All blocks of the grid; false when one gave up.
 __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, unsigned* status) {
@@ -88,14 +99,9 @@ __global__ void __launch_bounds__(kRk4Threads) k_rk4_grid(Rk4Args a) {
         AT acc[1];
         gather::accumulate<R, REALV ? gather::kReal : gather::kComplex, true, W1, 1, true>(a.v, st, sg, ell, (uint32_t)j,
                                                                                          x, 1, 0, 1, acc);
-        CT kv;
-        if constexpr (std::is_same<R, float>::value) {
-          gather::combine<0>(&kv, acc[0].total(), make_float2(0.f, -1.f), make_float2(0.f, 0.f));
-          rk4_stage_element<CT, float>(a.psi, a.acc, out, a.dt, j, kv, stage);
-        } else {
-          gather::combine<0>(&kv, acc[0].total(), make_double2(0.0, -1.0), make_double2(0.0, 0.0));
-          rk4_stage_element<CT, double>(a.psi, a.acc, out, a.dt, j, kv, stage);
-        }
+        const CT kv = minus_i(acc[0].total());
+        using S = typename std::conditional<std::is_same<R, float>::value, float, double>::type;
+        rk4_stage_element<CT, S>(a.psi, a.acc, out, a.dt, j, kv, stage);
       }
       if (step + 1 == a.nsteps && stage == 4) return;
       target += gridDim.x;
@@ -108,8 +114,10 @@ __global__ void __launch_bounds__(kRk4Threads) k_rk4_grid(Rk4Args a) {
 // ComplexF64 with real values; longer rows leave too few blocks resident.
 constexpr int kRk4ListMax = 64;
 
+// Seven blocks an SM hold 2^17 elements (double-float without the limit: 12 spins 1329, but 17
+// 5728 for 4276, its rows then without room).
 template <typename R, bool REALV>
-__global__ void __launch_bounds__(kRk4Threads) k_rk4_list(Rk4Args a, int cap) {
+__global__ void __launch_bounds__(kRk4Threads, 7) k_rk4_list(Rk4Args a, int cap) {
   using CT = typename gather::Cx<R>::T;
   using AT = typename gather::AccOf<R>::T;
   using ET = typename gather::Ell<R, REALV>::T;
@@ -148,6 +156,7 @@ __global__ void __launch_bounds__(kRk4Threads) k_rk4_list(Rk4Args a, int cap) {
     }
     own = p = static_cast<const CT*>(a.psi)[j];
   }
+  const int ne_warp = __reduce_max_sync(~0u, ne);
   const S dt = (S)a.dt;
   unsigned target = 0;
   for (int step = 0; step < a.nsteps; ++step) {
@@ -160,20 +169,29 @@ __global__ void __launch_bounds__(kRk4Threads) k_rk4_list(Rk4Args a, int cap) {
           acc.set(d, own);
         else
           acc.zero();
-        for (int e = 0; e < ne; e += 8) {
+        for (int e = 0; e < ne_warp; e += 8) {
           CT u[8];
 #pragma unroll
           for (int k = 0; k < 8; ++k)
             if (e + k < ne) u[k] = __ldcg(x + idx[(e + k) * kRk4Threads]);
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            if (e + k < ne) acc.mac(vals[(e + k) * kRk4Threads], u[k]);
+          for (int k = 0; k < 8; ++k) {
+            if constexpr (std::is_same<R, double>::value) {
+              if (e + k < ne) acc.mac(vals[(e + k) * kRk4Threads], u[k]);
+            } else {
+              // a loop of at most one turn stays a branch: the twenty (double-float) or
+              // eight instructions of an entry that no thread of the warp has are
+              // skipped; two FP64 ones are the faster under a predicate
+              int turn = e + k < ne_warp;
+              while (turn != 0) {
+                if (e + k < ne) acc.mac(vals[(e + k) * kRk4Threads], u[k]);
+                turn = 0;
+                asm volatile("" : "+r"(turn));
+              }
+            }
+          }
         }
-        CT kv;
-        if constexpr (std::is_same<R, float>::value)
-          gather::combine<0>(&kv, acc.total(), make_float2(0.f, -1.f), make_float2(0.f, 0.f));
-        else
-          gather::combine<0>(&kv, acc.total(), make_double2(0.0, -1.0), make_double2(0.0, 0.0));
+        const CT kv = minus_i(acc.total());
         // the stage combination (rk4_stage.cuh), psi and the sum in registers
         if (stage == 4) {
           const S c = dt / (S)6;
