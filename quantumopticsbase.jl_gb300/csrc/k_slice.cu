@@ -196,20 +196,19 @@ __device__ __forceinline__ int fixed_point(float v, int e) {
   const int f = sh >= 0 ? (int)(m << sh) : sh > -32 ? (int)(m >> -sh) : 0;
   return __float_as_int(v) < 0 ? -f : f;
 }
-// the lowest signed digit taken off f
-__device__ __forceinline__ int take_digit(long long& f) {
-  const int d = (int)(signed char)(int)f;
-  f = (f - d) >> 8;
-  return d;
+// All signed digits of f at once: f + sum 128 256^s has the bytes d_s + 128.
+__device__ __forceinline__ uint2 digit_bytes(long long f) {
+  const unsigned long long g = (unsigned long long)f + 0x8080808080808080ull;
+  return make_uint2((uint32_t)g, (uint32_t)(g >> 32));
 }
-__device__ __forceinline__ int take_digit(int& f) {
-  const int d = (int)(signed char)f;
-  f = (f - d) >> 8;
-  return d;
+__device__ __forceinline__ uint2 digit_bytes(int f) { return make_uint2((uint32_t)f + 0x80808080u, 0u); }
+// digits b of p and q, as two bytes (of d + 128)
+__device__ __forceinline__ uint32_t digit_pair(uint2 p, uint2 q, int b) {
+  return __byte_perm(b < 4 ? p.x : p.y, b < 4 ? q.x : q.y, (b & 3) | (((b & 3) + 4) << 4));
 }
-// small integer -> float bits: the mantissa of 1.5 2^23 + d
-__device__ __forceinline__ uint32_t small_float(int d) {
-  return __float_as_uint(__int_as_float(0x4b400000 + d) - 12582912.f);
+// digit b as the bits of a float: 2^23 + d + 128, less 2^23 + 128, exact
+__device__ __forceinline__ uint32_t digit_float(uint2 p, int b) {
+  return __float_as_uint(__uint_as_float(__byte_perm(b < 4 ? p.x : p.y, 0x4b000000u, 0x7440 | (b & 3))) - 8388736.f);
 }
 
 __device__ __forceinline__ double2 as_value(double2 v) { return v; }
@@ -254,20 +253,25 @@ __global__ void __launch_bounds__(split_threads(ROWS)) k_slice_split(const IN* _
   auto stage = [&](int b0) {  // k steps b0 .. of the chunk
     const int nk = min(sub, nks - b0) * 16;
     __syncthreads();
-    for (int i = threadIdx.x; i < H * nk; i += kSlSplit) {
-      int v, k;
-      if (kfast) {
-        v = i / nk;
-        k = i - v * nk;
-      } else {
-        k = i / H;
-        v = i - k * H;
+    // four elements of a thread in flight
+    for (int i0 = threadIdx.x; i0 < H * nk; i0 += 4 * kSlSplit) {
+      C2 val[4];
+      int at[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = i0 + u * kSlSplit;
+        val[u].x = val[u].y = 0;
+        at[u] = -1;
+        if (i >= H * nk) continue;
+        const int q = i / (kfast ? nk : H), r = i - q * (kfast ? nk : H);
+        const int v = kfast ? q : r, k = kfast ? r : q;
+        const int64_t kg = k0 + b0 * 16 + k;
+        at[u] = v * pitch + k;
+        if (off[v] >= 0 && kg < n) val[u] = as_value(x[off[v] + kg * es]);
       }
-      const int64_t kg = k0 + b0 * 16 + k;
-      C2 val;
-      val.x = val.y = 0;
-      if (off[v] >= 0 && kg < n) val = as_value(x[off[v] + kg * es]);
-      t[v * pitch + k] = val;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (at[u] >= 0) t[at[u]] = val[u];
     }
     __syncthreads();
     return nk;
@@ -315,18 +319,24 @@ __global__ void __launch_bounds__(split_threads(ROWS)) k_slice_split(const IN* _
       const bool im = INTER ? (r & 1) : r >= H;
       uint32_t w[S][INTER ? 2 : 4];
 #pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        const C2 a = t[v * pitch + kc * 8 + 2 * p], b = t[v * pitch + kc * 8 + 2 * p + 1];
-        auto fa = fixed_point<S>(im ? a.y : a.x, ex[v]), fb = fixed_point<S>(im ? b.y : b.x, ex[v]);
-        if (skip) fa = fb = 0;
+      for (int p = 0; p < 4; p += 2) {
+        uint2 g[4];
 #pragma unroll
-        for (int s = S - 1; s >= 0; --s) {
-          const int da = take_digit(fa), db = take_digit(fb);
+        for (int e = 0; e < 4; ++e) {
+          const C2 c = t[v * pitch + kc * 8 + 2 * p + e];
+          auto f = fixed_point<S>(im ? c.y : c.x, ex[v]);
+          if (skip) f = 0;
+          g[e] = digit_bytes(f);
+        }
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+          const int d = S - 1 - s;
           if constexpr (INTER) {
-            const uint32_t two = ((uint32_t)da & 0xffu) | (((uint32_t)db & 0xffu) << 8);
-            w[s][p >> 1] = (p & 1) ? w[s][p >> 1] | (two << 16) : two;
-          } else {
-            w[s][p] = __byte_perm(small_float(da), small_float(db), 0x7632);  // bf16: the upper half of a float
+            w[s][p >> 1] =
+                __byte_perm(digit_pair(g[0], g[1], d), digit_pair(g[2], g[3], d), 0x5410) ^ 0x80808080u;
+          } else {  // bf16: the upper half of a float
+            w[s][p] = __byte_perm(digit_float(g[0], d), digit_float(g[1], d), 0x7632);
+            w[s][p + 1] = __byte_perm(digit_float(g[2], d), digit_float(g[3], d), 0x7632);
           }
         }
       }
@@ -843,9 +853,12 @@ void run_split(const IN* x, int64_t n, int64_t es, const TcColMap& map, int64_t 
                unsigned char* out, int* exps, int* flags, cudaStream_t s, bool pdl) {
   const int nch = (nkb + kSlChunk - 1) / kSlChunk;
   auto kern = k_slice_split<FORM, ROWS, INTER, IN>;
-  // k steps staged at a time: the chunk, or half of it where 64 rows of 16 bytes are too many
-  const int sub = ROWS / 2 * sizeof(typename Sl<FORM>::V) <= 512 ? std::min(nkb, kSlChunk) : std::min(nkb, kSlChunk / 2);
-  const size_t smem = (size_t)(ROWS / 2) * (sub * 16 + 1) * sizeof(typename Sl<FORM>::V);
+  // k steps staged at a time: the chunk where it fits beside the tile's tables, otherwise half
+  // of it, read once for the largest components and again for the digits
+  auto bytes = [](int k) { return (size_t)(ROWS / 2) * (k * 16 + 1) * sizeof(typename Sl<FORM>::V); };
+  int sub = std::min(nkb, kSlChunk);
+  if (bytes(sub) > 226 * 1024) sub = kSlChunk / 2;
+  const size_t smem = bytes(sub);
   QOB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   launch_kernel(pdl, kern, dim3((unsigned)tiles, (unsigned)nch), (unsigned)split_threads(ROWS), smem, s, x, n, es, map, nvec, nkb,
                 es == 1 ? 1 : 0, sub, out, exps, flags);
