@@ -175,7 +175,7 @@ int qob_op_lazysum(qob_ctx* ctx, int64_t m, int64_t n, int nterms, const double*
  * to bras and operator rows (RIGHT: the same transform of the row with the two
  * phase vectors swapped, as the reference's conj / opposite-sign / conj
  * sequence gives); it may be a term of a LazySum or a factor of a LazyProduct.
- * Power-of-two axes use a radix-2 FFT, other lengths a direct DFT. */
+ * Power-of-two axes from 8 use an FFT, other lengths a direct DFT. */
 int qob_op_fft(qob_ctx* ctx, int nsub, const int64_t* shape, int naxes, const int64_t* axes, const int* sign,
                const double* before, const double* after, qob_op** out);
 

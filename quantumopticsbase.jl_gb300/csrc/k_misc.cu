@@ -132,8 +132,8 @@ __global__ void __launch_bounds__(128) k_dense(const CT* __restrict__ a, int64_t
 }
 
 // Double-float forms (ComplexF64 data, QOB_C128X): the operator factor is
-// stored as (re hi, re lo, im hi, im lo) quadruples, x arrives split the same
-// way (k_ff_split), the sums are FP32 pairs, joined to double for the FP64
+// stored as (re hi, re lo, im hi, im lo) quadruples, x arrives as (re hi, im hi,
+// re lo, im lo) (k_ff_split), the sums are FP32 pairs, joined to double for the FP64
 // alpha / beta epilogue (or for the partial sums of a split product).
 __device__ __forceinline__ double2 ff_total(const gather::AccFF& acc) {
   return make_double2(gather::ff_join(acc.rh, acc.rl), gather::ff_join(acc.ih, acc.il));
