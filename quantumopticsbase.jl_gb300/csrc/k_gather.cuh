@@ -1047,14 +1047,19 @@ void launch_j(const GatherView& v, const SiteTable& st, const void* x, int64_t x
   auto kern = k_gather_j<R, VM, SQUARE, W1, TC, BMODE>;
   allow_smem(kern, smem);
   int threads = v.block > 0 ? v.block : kThreads;
-  if (v.block == 0 && smem <= 4096) {
-    // Few blocks an SM and little to stage: smaller blocks share the work out more
-    // evenly.  A sparse operator of 4096 rows, ComplexF64, us with 256 threads -> by this
-    // rule: 8 vectors 11.1 -> 9.8, 100 19.1 -> 15.1, 251 32.3 -> 29.6 (512 blocks of 256 are
-    // four on some SMs and three on others); from 8 blocks an SM on, 500 vectors, 55.9 either way.
+  if ((std::is_same<R, double>::value || !W1) && v.block == 0 && smem <= 4096) {
+    // A few blocks an SM and little to stage: smaller blocks share the work out more
+    // evenly.  A sparse operator of 4096 rows, us with 256 threads -> by this rule:
+    // ComplexF64 100 vectors 19.1 -> 15.1, 256 29.4 -> 26.6, ComplexF32 256 8.9 -> 8.3 (512 blocks
+    // of 256 are four on some SMs and three on others); from 8 blocks an SM on, 500 vectors, 55.9
+    // either way; double-float 251 33.8 -> 29.4; 2048 states of several groups, 160 kets,
+    // ComplexF64 17.0 -> 13.8, but double-float 400 22.0 -> 23.4 (left out).  Not below a block an
+    // SM: fewer threads then only stage longer (512 states, one ket 2.7 -> 3.2).
     const int sms = current_sms();
     const int64_t sets = (ncols + (int64_t)TC * ls - 1) / ((int64_t)TC * ls);
-    while (threads > 64 && (v.m * ls + threads - 1) / threads * sets < 8 * (int64_t)sms) threads /= 2;
+    auto blocks = [&]() { return (v.m * ls + threads - 1) / threads * sets; };
+    if (blocks() >= sms)
+      while (threads > 64 && blocks() < 8 * (int64_t)sms) threads /= 2;
   }
   const int64_t jpb = threads / ls;  // output indices per block
   const unsigned gx = (unsigned)((v.m + jpb - 1) / jpb);
