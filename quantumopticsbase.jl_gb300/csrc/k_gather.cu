@@ -21,7 +21,6 @@ extern template void dispatch<DF>(const GatherView&, const SiteTable&, int, cons
 
 namespace {
 
-constexpr int kGroupsPerLaunch = 256;  // 256 * sizeof(GGroup) = 44 KB of shared memory
 
 // (hi, lo) float pair of a double: hi rounded to nearest, lo = the rest (not hot)
 __device__ __forceinline__ float2 split_rn(double v) {

@@ -387,13 +387,14 @@ static std::vector<c128> eval_slots(const GatherHost& H, const std::vector<TermC
 // stored entry made from the same contributions (so that re-evaluated
 // coefficients keep them equal).  Two 16-byte records per group: the groups that
 // touch the bits below the block of
-// indices per thread first, real groups before imaginary ones.
+// indices per thread first, real groups before imaginary ones.  Plans whose groups take
+// several launches keep the other kernels: the records and their four ranges are one launch's.
 static void build_flip_records(GatherPlan& gp, const GatherHost& H, const std::vector<GGroup>& descs,
                                const std::vector<int>& desc_group, bool store_real) {
   const uint32_t kLow = (uint32_t)flip_block(gp.precision, gp.ff) - 1;
   gp.multi = false;
   gp.two_runs = false;
-  if (!H.S.square || !store_real || descs.empty() || (gp.m & kLow) != 0) return;
+  if (!H.S.square || !store_real || descs.empty() || descs.size() > (size_t)kGroupsPerLaunch || (gp.m & kLow) != 0) return;
   struct Rec {
     int order;
     int4 row, flip;

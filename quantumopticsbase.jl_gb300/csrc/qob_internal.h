@@ -156,6 +156,9 @@ struct SiteTable {
   uint64_t mdout[kMaxSites];
 };
 
+// groups of one gather launch: 256 * sizeof(GGroup) = 44 KB of shared memory
+constexpr int kGroupsPerLaunch = 256;
+
 // consecutive output indices per thread of k_gather_m
 constexpr int flip_block(int precision, bool ff) { return precision == QOB_C64 && !ff ? 4 : 2; }
 
