@@ -9,20 +9,27 @@
 // S signed 8-bit digits of a fixed-point number (Ozaki, Ogita, Oishi & Rump 2012,
 // "Error-free transformations of matrix multiplication"): row i of the matrix
 // relative to 2^ea(i), the power of two above its largest component, vector c
-// relative to 2^ex(c), both per chunk of 256 contracted indices.  The product of
-// two digits is an integer of at most 2^14 and a chunk's sum of the pairs (i, j)
-// with i + j = d at most 256 (d + 1) 2^14: exact in an FP32 accumulator for d <= 3,
-// and beyond that rounding in the accumulator is below 2^-56 of the largest
-// term.  The accumulators of the S diagonals d = 0 .. S - 1 are added as 64-bit
-// integers and rounded once.  The digits:
-//   ComplexF64    S = 8: 62 bits below each row's and vector's largest component
-//                 (a component down to 2^-9 of it keeps all its 53 bits);
-//   double-float  S = 7: 54 bits (its components carry 48);
-//   ComplexF32    S = 4: 30 bits (down to 2^-6 all 24).
-// A vector tile (or matrix) with a component that is not finite, with exponents
-// far from 1 or with a nonzero component below 2^-kGrade of the largest is left to
-// the FMA arithmetic of the form: the split kernel flags the tile, the GEMM does
-// not store it and k_slice_fallback computes it.
+// relative to 2^ex(c), both per chunk of at most 256 contracted indices, 8 S - 2 bits
+// below it and truncated there.  The pairs (i, j) of digits with i + j = d < S are summed in
+// one FP32 accumulator, a diagonal, as integers; the S diagonals are added as 64-bit
+// integers and rounded once.  S = 8 in ComplexF64 (62 bits) and double-float, 5 in
+// ComplexF32 (38 bits).
+//
+// What the digits leave out is small against a row's and a vector's largest
+// components, and the products of those may be absent from a sum: a product is made of
+// digits only where a bound says that nothing is lost.  Per row or vector and chunk the split
+// kernel keeps the sum of the magnitudes, of the digits squared, and how many
+// components reach 2^-1 .. 2^-6 of the power of two.  The first two bound the error
+// (digit_error: the truncation of either side, the diagonals from S on; nothing rounds in an
+// accumulator below 2^24), the counts bound sum |a| |x| from below (overlap).  The error has to be
+// at most 2^-24 of that in ComplexF32, 2^-48 in double-float and 2^-50 in ComplexF64,
+// for every row, vector and chunk, Re and Im apart: no more than the bound of a chain of
+// multiply-adds over 4 terms, and the counts ask for more.  A tile of vectors that fails (graded
+// ones, sparse ones, components that are not finite or far from 1) is left
+// to the FMA arithmetic of the form: the split kernel flags it, the GEMM does not
+// store it and k_slice_fallback computes it.  A matrix that fails with vectors of ones has no
+// planes.  Gaussian entries (matrices of 32 to 4096 rows) reach 0.2 of the limit in ComplexF32
+// and double-float and 0.7 in ComplexF64, and 650 of the 1024 that keep a diagonal exact.
 //
 // Layout.  The complex product is one real GEMM as in k_tc32.cu: rows 2i, 2i + 1 of
 // a 128-row tile hold Re and Im of matrix row i, rows j and BN/2 + j of a BN-row
@@ -65,11 +72,14 @@ namespace qob {
 
 namespace {
 
-constexpr int kSlChunk = 16;      // k steps of 16 in a chunk
+constexpr int kSlChunk = 16;      // k steps of 16 in a chunk, at most
 constexpr int kSlRows = 128;      // real matrix rows of a tile
 constexpr int kSlPolls = 1 << 21;
 constexpr unsigned kSlErrTimeout = 1u;
-constexpr int kGrade = 40;        // nonzero components this far (2^-40) below the largest are left to the FMA form
+
+// The chunks of nkb k steps are of equal length but for one step: chunk c is the k
+// steps from chunk_start(c) to chunk_start(c + 1).
+__host__ __device__ inline int chunk_start(int c, int nkb, int nch) { return (int)((int64_t)c * nkb / nch); }
 
 __device__ __forceinline__ uint32_t saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void bar_init(uint64_t* b, unsigned n) {
@@ -144,21 +154,18 @@ struct Sl<QOB_C128> {
   static constexpr int S = 8;
   using V = double2;  // vectors
   using M = double2;  // the stored matrix
-  using F = long long;
 };
 template <>
 struct Sl<QOB_C128X> {
-  static constexpr int S = 7;
+  static constexpr int S = 8;
   using V = double2;
   using M = float4;
-  using F = long long;
 };
 template <>
 struct Sl<QOB_C64> {
-  static constexpr int S = 4;
+  static constexpr int S = 5;
   using V = float2;
   using M = float2;
-  using F = int;
 };
 template <int S>
 constexpr int kBits = 8 * S - 2;
@@ -188,12 +195,12 @@ __device__ __forceinline__ long long fixed_point(double v, int e) {
   return __double2hiint(v) < 0 ? -f : f;
 }
 template <int S>
-__device__ __forceinline__ int fixed_point(float v, int e) {
+__device__ __forceinline__ long long fixed_point(float v, int e) {
   const uint32_t hi = mag_hi(v);
   const int ev = (int)(hi >> 23);
   const uint32_t m = (hi & 0x7fffffu) | (ev ? 0x800000u : 0u);
   const int sh = kBits<S> - 24 - (e - ((ev ? ev : 1) - 126));
-  const int f = sh >= 0 ? (int)(m << sh) : sh > -32 ? (int)(m >> -sh) : 0;
+  const long long f = sh >= 0 ? (long long)m << sh : sh > -32 ? (long long)(m >> -sh) : 0;
   return __float_as_int(v) < 0 ? -f : f;
 }
 // All signed digits of f at once: f + sum 128 256^s has the bytes d_s + 128.
@@ -201,7 +208,6 @@ __device__ __forceinline__ uint2 digit_bytes(long long f) {
   const unsigned long long g = (unsigned long long)f + 0x8080808080808080ull;
   return make_uint2((uint32_t)g, (uint32_t)(g >> 32));
 }
-__device__ __forceinline__ uint2 digit_bytes(int f) { return make_uint2((uint32_t)f + 0x80808080u, 0u); }
 // digits b of p and q, as two bytes (of d + 128)
 __device__ __forceinline__ uint32_t digit_pair(uint2 p, uint2 q, int b) {
   return __byte_perm(b < 4 ? p.x : p.y, b < 4 ? q.x : q.y, (b & 3) | (((b & 3) + 4) << 4));
@@ -217,6 +223,39 @@ __device__ __forceinline__ double2 as_value(float4 v) {  // (re hi, re lo, im hi
   return make_double2((double)v.x + (double)v.y, (double)v.z + (double)v.w);
 }
 
+// What a row of the matrix or a vector tells about a chunk, the worst over the rows
+// (Re and Im each one) of a tile or of the whole matrix.  In units of 2^e, the power of two above the
+// row's largest component, |v| its components' magnitudes:
+struct SliceSide {
+  float n1;     // sum of |v|, at most
+  float t;      // sqrt(sum of all digits squared) / 128, at most
+  int c[6];     // components with |v| >= 1/2, 1/4, .. 1/64, at least
+};
+constexpr int kLevels = 6;
+
+// Error of the digit products allowed, in 2^-kBits of sum |a| |x|: a unit of the form
+// (2^-24, 2^-48), eight units of 2^-53 in ComplexF64.
+template <int FORM>
+constexpr float kSlLimit = FORM == QOB_C128 ? 4096.f : 16384.f;
+
+// A lower bound of sum |a| |x| over n indices, term (i, j): at least n less the components
+// of either side below their thresholds, 2^-(i + 1) and 2^-(j + 1), lie above both, and
+// the thresholds' differences add up to the largest that a component reaches.
+__host__ __device__ inline float overlap(const SliceSide& a, const SliceSide& x, int n, int i, int j) {
+  const float wi = 1.f / (float)(i + 1 < kLevels ? 4 << i : 2 << i), wj = 1.f / (float)(j + 1 < kLevels ? 4 << j : 2 << j);
+  const int both = a.c[i] + x.c[j] - n;
+  return both > 0 ? wi * wj * (float)both : 0.f;
+}
+// An upper bound of the digit products' error on n indices, in 2^-kBits of the row's times the vector's
+// power of two: each side's truncation, below 1, times the other's components, and the
+// diagonals from S on (|sum of d_i d_(S-i)| <= |a's digits| |x's digits|, the ones after it
+// 256 times smaller each).  Infinite where a diagonal's sum could leave 2^24, the
+// integers that an FP32 accumulator holds.
+__host__ __device__ inline float digit_error(const SliceSide& a, const SliceSide& x) {
+  const float t = a.t * x.t;
+  return t > 1024.f ? 3e38f : a.n1 + x.n1 + 1.01f * t;
+}
+
 __device__ __forceinline__ int64_t col_offset(const TcColMap& m, int64_t c) {
   if (m.s1 == 1 && m.s3 == 1) return c * m.st;
   const uint32_t cc = (uint32_t)c, s1 = (uint32_t)m.s1, s3 = (uint32_t)m.s3;
@@ -227,28 +266,36 @@ __device__ __forceinline__ int64_t col_offset(const TcColMap& m, int64_t c) {
 // Digit planes of one tile's chunk: ROWS / 2 vectors (columns of x, or rows of the
 // matrix with INTER) x up to 256 contracted indices.  blockIdx.x: tile, blockIdx.y:
 // chunk.  exps[(tile nch + chunk) ROWS / 2 + vector]: the power of two above its
-// largest component; flags[tile nch + chunk]: 1 where the tile is left to the FMA
-// form (its planes are zero then).  KFAST: threads read along the contracted index.
+// largest component.  flags[tile nch + chunk]: 1 where the tile is left to the FMA
+// form, by its exponents or, with the matrix's chunks in `other`, by the bounds above;
+// own[tile nch + chunk]: the tile's side of them.  kfast: threads read along the contracted index.
 constexpr int split_threads(int rows) { return rows == 32 ? 512 : 1024; }
 template <int FORM, int ROWS, bool INTER, typename IN>
 __global__ void __launch_bounds__(split_threads(ROWS)) k_slice_split(const IN* __restrict__ x, int64_t n, int64_t es, TcColMap map,
                                                      int64_t nvec, int nkb, int kfast, int sub,
-                                                     unsigned char* __restrict__ out,
-                                                     int* __restrict__ exps, int* __restrict__ flags) {
+                                                     unsigned char* __restrict__ out, int* __restrict__ exps,
+                                                     int* __restrict__ flags, const SliceSide* __restrict__ other,
+                                                     SliceSide* __restrict__ own) {
   constexpr int S = Sl<FORM>::S, H = ROWS / 2, kSlSplit = split_threads(ROWS);
   using C2 = decltype(as_value(IN{}));
   using T = decltype(C2{}.x);
   extern __shared__ __align__(16) unsigned char sl_smem[];
-  __shared__ int ex[H];
+  __shared__ int ex[H], some[H];  // some: bit 0: nonzero real parts, bit 1: imaginary ones
   __shared__ int bad;
   __shared__ int64_t off[H];
+  // per real row: components by their level, three counts of 10 bits a word, sum |v| in 2^-14, digits squared
+  __shared__ uint32_t cnt_hi[ROWS], cnt_lo[ROWS], sum1[ROWS], sum2[ROWS];
+  __shared__ SliceSide side;
+  __shared__ int worst1, worst2;
   pdl_enter();
-  const int kb0 = blockIdx.y * kSlChunk, nks = min(kSlChunk, nkb - kb0);
+  const int nch = gridDim.y, kb0 = chunk_start(blockIdx.y, nkb, nch), nks = chunk_start(blockIdx.y + 1, nkb, nch) - kb0;
   const int64_t k0 = (int64_t)kb0 * 16;
   const int pitch = sub * 16 + 1;  // sub k steps are staged at a time
   C2* t = reinterpret_cast<C2*>(sl_smem);  // [vector][k]
   const int64_t v0 = (int64_t)blockIdx.x * H;
-  if (threadIdx.x == 0) bad = 0;
+  if (threadIdx.x == 0) bad = worst1 = worst2 = 0;
+  if (threadIdx.x < kLevels) side.c[threadIdx.x] = kSlChunk * 16;
+  if (threadIdx.x < ROWS) cnt_hi[threadIdx.x] = cnt_lo[threadIdx.x] = sum1[threadIdx.x] = sum2[threadIdx.x] = 0u;
   if (threadIdx.x < H) off[threadIdx.x] = v0 + threadIdx.x < nvec ? col_offset(map, v0 + threadIdx.x) : -1;
   auto stage = [&](int b0) {  // k steps b0 .. of the chunk
     const int nk = min(sub, nks - b0) * 16;
@@ -281,33 +328,30 @@ __global__ void __launch_bounds__(split_threads(ROWS)) k_slice_split(const IN* _
   static_assert(PER * H == kSlSplit && PER <= 32, "threads of a vector in one warp");
   {
     const int v = threadIdx.x / PER, part = threadIdx.x % PER;
-    uint32_t mx = 0u, mn = 0xffffffffu;
+    uint32_t mx = 0u, nonzero = 0u;
     for (int b0 = 0; b0 < nks; b0 += sub) {
       const int nk = stage(b0);
       for (int k = part; k < nk; k += PER) {
         const C2 c = t[v * pitch + k];
         mx = max(mx, max(mag_hi(c.x), mag_hi(c.y)));
-        if (is_nonzero(c.x)) mn = min(mn, mag_hi(c.x));
-        if (is_nonzero(c.y)) mn = min(mn, mag_hi(c.y));
+        nonzero |= (is_nonzero(c.x) ? 1u : 0u) | (is_nonzero(c.y) ? 2u : 0u);
       }
     }
 #pragma unroll
     for (int w = PER / 2; w > 0; w >>= 1) {
       mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, w));
-      mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, w));
+      nonzero |= __shfl_xor_sync(0xffffffffu, nonzero, w);
     }
     if (part == 0) {
-      const bool any = mn != 0xffffffffu;
-      const int e = any ? exp_above<T>(mx) : 0;
+      const int e = nonzero ? exp_above<T>(mx) : 0;
       ex[v] = e;
-      if (any && (e > kExpMax<T> || e < -kExpMax<T> || e - exp_above<T>(mn) > kGrade)) atomicExch(&bad, 1);
+      some[v] = (int)nonzero;
+      if (nonzero && (e > kExpMax<T> || e < -kExpMax<T>)) atomicExch(&bad, 1);
     }
   }
   __syncthreads();
-  const bool skip = bad != 0;
-  const int64_t tile = (int64_t)blockIdx.x * gridDim.y + blockIdx.y;
+  const int64_t tile = (int64_t)blockIdx.x * nch + blockIdx.y;
   if (threadIdx.x < H) exps[tile * H + threadIdx.x] = ex[threadIdx.x];
-  if (threadIdx.x == 0) flags[tile] = skip ? 1 : 0;
   for (int b0 = 0; b0 < nks; b0 += sub) {
     const int nk = sub < nks ? stage(b0) : nks * 16;  // staged already when it is all of the chunk
     // 8 contracted indices of one real row per task: a store of 16 (INTER: 8) bytes per plane
@@ -318,15 +362,22 @@ __global__ void __launch_bounds__(split_threads(ROWS)) k_slice_split(const IN* _
       const int v = INTER ? r >> 1 : r % H;
       const bool im = INTER ? (r & 1) : r >= H;
       uint32_t w[S][INTER ? 2 : 4];
+      unsigned long long levels = 0ull;
+      uint32_t n1 = 0u;
+      int n2 = 0;
 #pragma unroll
       for (int p = 0; p < 4; p += 2) {
         uint2 g[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const C2 c = t[v * pitch + kc * 8 + 2 * p + e];
-          auto f = fixed_point<S>(im ? c.y : c.x, ex[v]);
-          if (skip) f = 0;
+          const long long f = fixed_point<S>(im ? c.y : c.x, ex[v]);
+          const unsigned long long mag = f < 0 ? -f : f;
           g[e] = digit_bytes(f);
+          levels += 1ull << (10 * min(__clzll((long long)mag) - (64 - kBits<S>), kLevels));
+          n1 += (uint32_t)(mag >> (kBits<S> - 14));
+          const int lo = (int)(g[e].x ^ 0x80808080u), hi = (int)((g[e].y ^ 0x80808080u) & (S == 8 ? ~0u : 0xffu));
+          n2 = __dp4a(hi, hi, __dp4a(lo, lo, n2));
         }
 #pragma unroll
         for (int s = 0; s < S; ++s) {
@@ -349,7 +400,52 @@ __global__ void __launch_bounds__(split_threads(ROWS)) k_slice_split(const IN* _
         else
           *reinterpret_cast<uint4*>(q + s * (ROWS * kRow)) = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
       }
+      atomicAdd(&cnt_hi[r], (uint32_t)levels & 0x3fffffffu);
+      atomicAdd(&cnt_lo[r], (uint32_t)(levels >> 30) & 0x3fffffffu);
+      atomicAdd(&sum1[r], n1);
+      atomicAdd(&sum2[r], (uint32_t)n2);
     }
+  }
+  __syncthreads();
+  // the worst of the rows that are not zero
+  const int valid = (int)min((int64_t)nks * 16, n - k0);
+  if (threadIdx.x < ROWS) {
+    const int r = threadIdx.x, v = INTER ? r >> 1 : r % H;
+    const bool im = INTER ? (r & 1) : r >= H;
+    const bool on = (some[v] >> (im ? 1 : 0)) & 1;
+    int c = 0;
+#pragma unroll
+    for (int i = 0; i < kLevels; ++i) {
+      c += (int)(((i < 3 ? cnt_hi[r] : cnt_lo[r]) >> (10 * (i % 3))) & 0x3ffu);
+      const int least = __reduce_min_sync(0xffffffffu, on ? c : kSlChunk * 16);
+      if ((r & 31) == 0) atomicMin(&side.c[i], least);
+    }
+    const int most1 = __reduce_max_sync(0xffffffffu, on ? (int)sum1[r] + valid : 0);  // each of its terms rounded up
+    const int most2 = __reduce_max_sync(0xffffffffu, on ? (int)sum2[r] : 0);
+    if ((r & 31) == 0) {
+      atomicMax(&worst1, most1);
+      atomicMax(&worst2, most2);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  SliceSide mine;
+  mine.n1 = (float)worst1 * (1.f / 16384.f);
+  mine.t = sqrtf((float)worst2) * (1.f / 128.f);
+#pragma unroll
+  for (int i = 0; i < kLevels; ++i) mine.c[i] = side.c[i];
+  bool left = bad != 0;
+  if (other) {
+    const SliceSide a = other[blockIdx.y];
+    float least = 0.f;
+    for (int q = threadIdx.x; q < kLevels * kLevels; q += 32) least += overlap(a, mine, valid, q / kLevels, q % kLevels);
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) least += __shfl_xor_sync(0xffffffffu, least, w);
+    left |= digit_error(a, mine) > kSlLimit<FORM> * least;
+  }
+  if (threadIdx.x == 0) {
+    flags[tile] = left ? 1 : 0;
+    if (own) own[tile] = mine;
   }
 }
 
@@ -360,7 +456,7 @@ struct SlCfg {
   static constexpr int kSets = 2 * kCols <= 512 ? 2 : 1;     // sets in the tensor memory
   // k steps of a widened buffer (one rendezvous and its commits, ~300 cycles, beside
   // 80 or more per MMA) and of a stage
-  static constexpr int kG = S == 4 ? 2 : 1, kKs = 2;
+  static constexpr int kG = S < 8 ? 2 : 1, kKs = 2;
   static constexpr int kA = S * kSlRows * 16, kB = S * BN * 32;  // one k step: bytes of the M side, planes of the N side
   static constexpr int kWideStep = S * kSlRows * 32;             // one k step of the M side, widened
   static constexpr int kWide = kG * kWideStep;
@@ -382,7 +478,7 @@ struct SlCfg {
   static_assert(smem <= 227 * 1024, "shared memory of a block");
 };
 
-// H 2^(8 (S - 4)) + L: the sum of the diagonals in units of the last one's
+// H 2^32 + L (S = 8) or H (S = 5): the sum of the diagonals in units of the last one's
 struct Sum2 {
   long long h, l;
 };
@@ -393,13 +489,12 @@ __device__ __forceinline__ Sum2 add_diagonals(const uint32_t (&d)[S]) {
   r.h = in(0) * (1 << 24) + in(1) * (1 << 16) + in(2) * (1 << 8) + in(3);
   r.l = 0;
   if constexpr (S == 8) r.l = in(4) * (1 << 24) + in(5) * (1 << 16) + in(6) * (1 << 8) + in(7);
-  if constexpr (S == 7) r.l = in(4) * (1 << 16) + in(5) * (1 << 8) + in(6);
+  if constexpr (S == 5) r.h = r.h * (1 << 8) + in(4);  // at most 2^55: one part
   return r;
 }
-// the sum in units of 2^(e - 36 - 8 (S - 4)), rounded to nearest, without the FP64 pipe
-template <int S>
+// the sum of S = 8 in units of 2^(e - 68), rounded to nearest, without the FP64 pipe
 __device__ __forceinline__ double sum_to_double(Sum2 v, int e) {
-  constexpr int LB = 8 * (S - 4);               // bits of the low part's unit below the high one's
+  constexpr int LB = 32;                        // bits of the low part's unit below the high one's
   long long g = v.h + (v.l >> LB);              // floor
   unsigned long long f = (unsigned long long)v.l << (64 - LB);  // fraction, in units of 2^-64
   const bool neg = g < 0;
@@ -464,7 +559,7 @@ __global__ void __launch_bounds__(SlCfg<FORM, BN>::kThreads, 1)
   const int64_t u0 = (int64_t)blockIdx.x * per;
   const int nu = (int)(units - u0 < (int64_t)per ? units - u0 : (int64_t)per);
   const int ch_start = (int)(u0 % nch);
-  auto steps = [&](int ch) { return min(kSlChunk, nkb - ch * kSlChunk); };
+  auto steps = [&](int ch) { return chunk_start(ch + 1, nkb, nch) - chunk_start(ch, nkb, nch); };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < NA; ++s) {
@@ -526,7 +621,7 @@ __global__ void __launch_bounds__(SlCfg<FORM, BN>::kThreads, 1)
             stop = true;
             break;
           }
-          const int64_t kb = (int64_t)ch * kSlChunk + k;
+          const int64_t kb = chunk_start(ch, nkb, nch) + k;
           const uint32_t q = (uint32_t)min(KS, ks - k);
           bar_expect(&afull[sa], q * C::kA);
           bulk_copy(ring_a + (size_t)sa * C::kStageA, A + (mti * nkb + kb) * C::kA, q * C::kA, &afull[sa]);
@@ -638,7 +733,7 @@ __global__ void __launch_bounds__(SlCfg<FORM, BN>::kThreads, 1)
     // the vectors [h KQ, (h + 1) KQ): their real columns and, BN/2 on, their imaginary ones
     const int q4 = warp & 3, half = (warp - 3 - C::kWidenWarps) >> 2;
     constexpr int KQ = BN / 2 / (C::kAddWarps / 4);
-    constexpr int CG = S == 4 ? 4 : 2;  // columns at a time
+    constexpr int CG = S == 5 ? 4 : 2;  // columns at a time
     const uint32_t lane_addr = tmem + ((uint32_t)(q4 * 32) << 16);
     const int r = q4 * 32 + lane, il = r >> 1;
     const bool even = (lane & 1) == 0;
@@ -683,13 +778,13 @@ __global__ void __launch_bounds__(SlCfg<FORM, BN>::kThreads, 1)
           // even lane: Re y = Re a Re x - Im a Im x; odd lane: Im y = Im a Re x + Re a Im x
           o.h = __shfl_xor_sync(0xffffffffu, o.h, 1);
           a.h += even ? -o.h : o.h;
-          if constexpr (S > 4) {
+          if constexpr (S == 8) {
             o.l = __shfl_xor_sync(0xffffffffu, o.l, 1);
             a.l += even ? -o.l : o.l;
-            got[c] = sum_to_double<S>(a, er + __shfl_sync(0xffffffffu, ec, c0 + c));
+            got[c] = sum_to_double(a, er + __shfl_sync(0xffffffffu, ec, c0 + c));
           } else {
             const int e = __shfl_sync(0xffffffffu, ec, c0 + c);
-            got[c] = __ll2float_rn(a.h) * __int_as_float((er - 18 + 127) << 23) * __int_as_float((e - 18 + 127) << 23);
+            got[c] = __ll2float_rn(a.h) * __int_as_float((er - 22 + 127) << 23) * __int_as_float((e - 22 + 127) << 23);
           }
         }
 #pragma unroll
@@ -850,18 +945,19 @@ __global__ void __launch_bounds__(128) k_slice_fallback(const typename Sl<FORM>:
 
 template <int FORM, int ROWS, bool INTER, typename IN>
 void run_split(const IN* x, int64_t n, int64_t es, const TcColMap& map, int64_t nvec, int64_t tiles, int nkb,
-               unsigned char* out, int* exps, int* flags, cudaStream_t s, bool pdl) {
+               unsigned char* out, int* exps, int* flags, const SliceSide* other, SliceSide* own, cudaStream_t s,
+               bool pdl) {
   const int nch = (nkb + kSlChunk - 1) / kSlChunk;
   auto kern = k_slice_split<FORM, ROWS, INTER, IN>;
   // k steps staged at a time: the chunk where it fits beside the tile's tables, otherwise half
   // of it, read once for the largest components and again for the digits
   auto bytes = [](int k) { return (size_t)(ROWS / 2) * (k * 16 + 1) * sizeof(typename Sl<FORM>::V); };
   int sub = std::min(nkb, kSlChunk);
-  if (bytes(sub) > 226 * 1024) sub = kSlChunk / 2;
+  if (bytes(sub) > 220 * 1024) sub = kSlChunk / 2;
   const size_t smem = bytes(sub);
   QOB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   launch_kernel(pdl, kern, dim3((unsigned)tiles, (unsigned)nch), (unsigned)split_threads(ROWS), smem, s, x, n, es, map, nvec, nkb,
-                es == 1 ? 1 : 0, sub, out, exps, flags);
+                es == 1 ? 1 : 0, sub, out, exps, flags, other, own);
   QOB_LAUNCHED();
 }
 
@@ -891,6 +987,8 @@ void run_slices(const SliceDense& d, bool swap, const void* a, const void* xv, i
   const int64_t blocks = (units + per - 1) / per;
   const int smax = (int)((nch - 1) / per + 2);
   const int64_t tile = swap ? HM : H;  // vectors of a tile
+  const SlicePlanes& pl = swap ? d.nside : d.mside;
+  const SliceSide* sides = static_cast<const SliceSide*>(pl.sides.p);
   const size_t bbytes = (size_t)vt * nkb * (swap ? C::kA : C::kB), ebytes = (size_t)vt * nch * (tile + 1) * sizeof(int);
   unsigned char* w = static_cast<unsigned char*>(ws->get(slot, bbytes + ebytes));
   int* exps = reinterpret_cast<int*>(w + bbytes);
@@ -898,10 +996,9 @@ void run_slices(const SliceDense& d, bool swap, const void* a, const void* xv, i
   V* part = nullptr;
   if (per % nch != 0) part = static_cast<V*>(ws->get(slot + 1, (size_t)rtiles * smax * H * HM * sizeof(V)));
   if (swap)
-    run_split<FORM, kSlRows, true, V>(x, d.n, xes, xm, ncols, vt, nkb, w, exps, flags, s, pdl);
+    run_split<FORM, kSlRows, true, V>(x, d.n, xes, xm, ncols, vt, nkb, w, exps, flags, sides, nullptr, s, pdl);
   else
-    run_split<FORM, BN, false, V>(x, d.n, xes, xm, ncols, vt, nkb, w, exps, flags, s, pdl);
-  const SlicePlanes& pl = swap ? d.nside : d.mside;
+    run_split<FORM, BN, false, V>(x, d.n, xes, xm, ncols, vt, nkb, w, exps, flags, sides, nullptr, s, pdl);
   const unsigned char* mp = swap ? w : static_cast<const unsigned char*>(pl.planes.p);
   const unsigned char* np = swap ? static_cast<const unsigned char*>(pl.planes.p) : w;
   const int* me = swap ? exps : static_cast<const int*>(pl.exps.p);
@@ -938,22 +1035,47 @@ void build_slices(SliceDense& d, bool swap, const void* a, cudaStream_t s) {
   pl.exps.alloc((size_t)tiles * nch * (half + 1) * sizeof(int));
   int* exps = static_cast<int*>(pl.exps.p);
   int* flags = exps + tiles * nch * half;
+  DeviceBuf own;
+  own.alloc((size_t)(tiles * nch) * sizeof(SliceSide));
+  auto* tile_sides = static_cast<SliceSide*>(own.p);
   TcColMap map;  // "vectors" = matrix rows, one element apart; contracted index = column, m apart
   map.st = 1;
   const auto* m = static_cast<const typename Sl<FORM>::M*>(a);
   if (swap)
     run_split<FORM, kSwapBN, false, typename Sl<FORM>::M>(m, d.n, d.m, map, d.m, tiles, d.nkb,
-                                                          static_cast<unsigned char*>(pl.planes.p), exps, flags, s, false);
+                                                          static_cast<unsigned char*>(pl.planes.p), exps, flags,
+                                                          nullptr, tile_sides, s, false);
   else
     run_split<FORM, kSlRows, true, typename Sl<FORM>::M>(m, d.n, d.m, map, d.m, tiles, d.nkb,
-                                                         static_cast<unsigned char*>(pl.planes.p), exps, flags, s, false);
+                                                         static_cast<unsigned char*>(pl.planes.p), exps, flags,
+                                                         nullptr, tile_sides, s, false);
   std::vector<int> f((size_t)(tiles * nch));
+  std::vector<SliceSide> q((size_t)(tiles * nch)), worst((size_t)nch);
   QOB_CUDA(cudaMemcpyAsync(f.data(), flags, f.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
+  QOB_CUDA(cudaMemcpyAsync(q.data(), tile_sides, q.size() * sizeof(SliceSide), cudaMemcpyDeviceToHost, s));
   QOB_CUDA(cudaStreamSynchronize(s));
   pl.state = 1;
   for (int v : f)
     if (v) pl.state = -1;
-  if (pl.state < 0) {
+  for (int ch = 0; ch < nch; ++ch) {
+    SliceSide& w = worst[(size_t)ch] = q[(size_t)ch];
+    for (int64_t t = 1; t < tiles; ++t) {
+      const SliceSide& o = q[(size_t)(t * nch + ch)];
+      w.n1 = std::max(w.n1, o.n1);
+      w.t = std::max(w.t, o.t);
+      for (int i = 0; i < kLevels; ++i) w.c[i] = std::min(w.c[i], o.c[i]);
+    }
+    // a matrix that fails even with vectors of ones is left to the FMA kernels at once
+    const int n = (int)std::min<int64_t>(d.n, (int64_t)chunk_start(ch + 1, d.nkb, nch) * 16) -
+                  chunk_start(ch, d.nkb, nch) * 16;
+    const SliceSide ones{0.5f * (float)n, 0.f, {n, n, n, n, n, n}};
+    float least = 0.f;
+    for (int k = 0; k < kLevels * kLevels; ++k) least += overlap(w, ones, n, k / kLevels, k % kLevels);
+    if (digit_error(w, ones) > kSlLimit<FORM> * least) pl.state = -1;
+  }
+  if (pl.state > 0) {
+    pl.sides.upload(worst.data(), worst.size() * sizeof(SliceSide));
+  } else {
     pl.planes = DeviceBuf();
     pl.exps = DeviceBuf();
   }

@@ -323,6 +323,7 @@ struct TcColMap {
 struct SlicePlanes {
   int state = 0;  // 0: not made, 1: ready, -1: the matrix is left to the FMA kernels
   DeviceBuf planes, exps;
+  DeviceBuf sides;  // per chunk, the worst of the rows (k_slice.cu, SliceSide)
 };
 struct SliceDense {
   int64_t m = 0, n = 0;
