@@ -131,23 +131,22 @@ void apply_plan(Context& ctx, Plan& P, c128 alpha, const void* x, int64_t xes, i
     }
     for (auto& d : P.dense) {
       // partial sums of a split product in slot ws (free here, as for the split input above);
-      // a double-float plan splits x into slot ws + 1 first
+      // a double-float plan splits x into slot ws + 1 first; digit planes use ws + 2 and
+      // ws + 3 (sub-plans run after), and the tiles they leave go to the FMA kernels
       const c128 ad = cmul(alpha, coefval(d.coef, P.root));
       const int form = P.ff ? QOB_C128X : P.precision;
       TcColMap xm, ym;
       xm.st = xcs;
       ym.st = ycs;
+      FmaGate gate;
       if (!(form == QOB_C64 ? ctx.fp32_tensor : ctx.fp64_tensor && !P.ff) && slices_pay(form, d.m, d.n, ncols, false) &&
-          slice_ready(d.sl, form, d.a.p, d.m, d.n, slice_swap(yes, ym, ncols), s)) {
-        launch_slices(d.sl, form, d.a.p, ad, x, xes, xm, b, y, yes, ym, ncols, s, &ctx.ws, ws,
-                      static_cast<unsigned*>(ctx.status.p), ctx.num_sms, ctx.pdl);
-        b = one;
-        continue;
-      }
+          slice_ready(d.sl, form, d.a.p, d.m, d.n, slice_swap(yes, ym, ncols), s))
+        gate = launch_slices(d.sl, form, ad, x, xes, xm, b, y, yes, ym, ncols, s, &ctx.ws, ws + 2,
+                             static_cast<unsigned*>(ctx.status.p), ctx.num_sms, ctx.pdl);
       const void* xin = x;
       if (P.ff) {
         void* xs = ctx.ws.get(ws + 1, (size_t)((P.n - 1) * xes + (ncols - 1) * xcs + 1) * 16);
-        launch_ff_split(x, P.n, ncols, xes, xcs, xs, s);
+        launch_ff_split(x, P.n, ncols, xes, xcs, xs, s, gate.any);
         xin = xs;
       }
       if (ctx.fp32_tensor && P.precision == QOB_C64 && !P.ff && d.m >= kDmmaMinK && d.n >= kDmmaMinK) {
@@ -156,7 +155,7 @@ void apply_plan(Context& ctx, Plan& P, c128 alpha, const void* x, int64_t xes, i
                         static_cast<unsigned*>(ctx.status.p), ctx.num_sms, ctx.pdl);
       } else {
         launch_dense(P.precision, d.a.p, d.m, d.n, ad, xin, xes, xcs, b, y, yes, ycs, ncols, s, &ctx.ws, ws, P.ff,
-                     ctx.fp64_tensor);
+                     ctx.fp64_tensor, gate);
       }
       b = one;
     }
@@ -196,30 +195,31 @@ void apply_plan(Context& ctx, Plan& P, c128 alpha, const void* x, int64_t xes, i
         const bool slices = !st.eye && !(form == QOB_C64 ? ctx.fp32_tensor : ctx.fp64_tensor && !P.ff) &&
                             slices_pay(form, st.dout, st.din, pcols, true) &&
                             slice_ready(st.sl, form, st.a.p, st.dout, st.din, slice_swap(s1 * out_es, ym, pcols), s);
-        const bool ffs = P.ff && !st.eye && !slices;
-        const void* sin = src;
-        if (ffs) {
-          const int64_t len_in = prod_range(cur, 0, cur.size());
-          void* xs = ctx.ws.get(ws + 2, (size_t)((len_in - 1) * ses + (ncols - 1) * scs + 1) * 16);
-          launch_ff_split(src, len_in, ncols, ses, scs, xs, s);
-          sin = xs;
-        }
+        const bool ffs = P.ff && !st.eye;
         // ComplexF32 dense factors on the tensor cores: one product with the
         // (before, after, ket) index triples as columns, contracted dimension din
         const bool tc = ctx.fp32_tensor && P.precision == QOB_C64 && !ffs && !st.eye && st.din >= kDmmaMinK &&
                         st.dout >= kDmmaMinK;
         auto mode_product = [&](c128 bk, void* out) {
           unsigned* status = static_cast<unsigned*>(ctx.status.p);
-          if (slices) {
-            launch_slices(st.sl, form, st.a.p, ak, sin, s1 * ses, xm, bk, out, s1 * out_es, ym, pcols, s, &ctx.ws, ws + 3,
-                          status, ctx.num_sms, ctx.pdl);
-          } else if (tc) {
+          FmaGate gate;
+          if (slices)
+            gate = launch_slices(st.sl, form, ak, src, s1 * ses, xm, bk, out, s1 * out_es, ym, pcols, s, &ctx.ws, ws + 3,
+                                 status, ctx.num_sms, ctx.pdl);
+          const void* sin = src;
+          if (ffs) {
+            const int64_t len_in = prod_range(cur, 0, cur.size());
+            void* xs = ctx.ws.get(ws + 2, (size_t)((len_in - 1) * ses + (ncols - 1) * scs + 1) * 16);
+            launch_ff_split(src, len_in, ncols, ses, scs, xs, s, gate.any);
+            sin = xs;
+          }
+          if (tc) {
             if (!st.tc.ready) tc_dense_build(st.tc, st.a.p, st.dout, st.din, s);
             launch_gemm_tc(st.tc, ak, sin, s1 * ses, xm, bk, out, s1 * out_es, ym, pcols, s, &ctx.ws, ws + 3, status,
                            ctx.num_sms, ctx.pdl);
           } else {
             launch_modek(P.precision, st.a.p, st.eye, s1, st.dout, st.din, s3, ak, sin, ses, scs, bk, out, out_es,
-                         out_cs, ncols, s, ffs, ctx.fp64_tensor);
+                         out_cs, ncols, s, ffs, ctx.fp64_tensor, gate);
           }
         };
         if (last) {

@@ -65,8 +65,13 @@ __global__ void k_build_diag(int64_t m, int ndg, const GGroup* __restrict__ dg,
 // lo, im lo: pairs as the packed FP32 instructions take them), element e of vector c at e * es + c * cs in both arrays.  Each
 // thread moves kSplitPer elements a block apart, their loads issued together.
 constexpr int kSplitPer = 4;
+template <bool GATED>
 __global__ void __launch_bounds__(256) k_ff_split(const double2* __restrict__ x, int64_t n, int64_t ncols,
-                                                  int64_t es, int64_t cs, float4* __restrict__ out) {
+                                                  int64_t es, int64_t cs, float4* __restrict__ out, const int* any) {
+  if constexpr (GATED) {
+    pdl_wait();
+    if (*any == 0) return;
+  }
   const int64_t total = n * ncols;
   const int64_t i0 = blockIdx.x * (int64_t)blockDim.x * kSplitPer + threadIdx.x;
   int64_t o[kSplitPer];
@@ -226,11 +231,13 @@ int gather_tile(const GatherPlan& g, int64_t ncols) {
   return tc;
 }
 
-void launch_ff_split(const void* x, int64_t n, int64_t ncols, int64_t es, int64_t cs, void* out, cudaStream_t s) {
+void launch_ff_split(const void* x, int64_t n, int64_t ncols, int64_t es, int64_t cs, void* out, cudaStream_t s,
+                     const int* any) {
   const int64_t total = n * ncols;
   if (total == 0) return;
   const unsigned blocks = (unsigned)((total + 256 * kSplitPer - 1) / (256 * kSplitPer));
-  k_ff_split<<<blocks, 256, 0, s>>>(static_cast<const double2*>(x), n, ncols, es, cs, static_cast<float4*>(out));
+  launch_kernel(any != nullptr, any ? k_ff_split<true> : k_ff_split<false>, dim3(blocks), 256u, 0, s,
+                static_cast<const double2*>(x), n, ncols, es, cs, static_cast<float4*>(out), any);
   QOB_LAUNCHED();
 }
 

@@ -10,6 +10,7 @@
 #include <algorithm>
 
 #include "k_gather.cuh"  // double-float helpers (ff_join, AccFF)
+#include "launch.cuh"
 #include "qob_internal.h"
 
 namespace qob {
@@ -75,20 +76,40 @@ __global__ void k_axpby(const CT* __restrict__ x, int64_t xes, int64_t xcs, CT* 
   *yp = mk<CT>(re, im);
 }
 
+// Kernels behind a gate: whether vector c of this call is one of theirs.
+__device__ __forceinline__ bool gate_open(const FmaGate& g, int64_t c) {
+  pdl_wait();
+  return *g.any != 0 && left_to_fma(g, g.c0 + c);
+}
+// f(i) for the output elements i < len of a vector: one a thread, or, behind a gate, as many
+// as its smaller grid leaves over.
+template <bool GATED, typename F>
+__device__ __forceinline__ void each_element(int64_t len, const FmaGate& gate, F f) {
+  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if constexpr (!GATED) {
+    if (i < len) f(i);
+  } else {
+    pdl_wait();
+    if (*gate.any == 0) return;
+    for (; i < len; i += (int64_t)gridDim.x * blockDim.x) f(i);
+  }
+}
+
 // Dense operator (m x n, column-major) times ncols vectors.  A thread owns one
 // row i and a tile of TC vectors (each A element it loads serves all of them);
 // blocks split the columns k into kchunks ranges so that a tall-skinny product
 // (one ket, m ~ 1000) still fills the GPU.  With one range the thread writes
 // alpha * acc + beta * y; otherwise it writes its partial sum to part[z][c][i]
 // and k_dense_reduce adds the ranges in order (deterministic) and combines.
-template <typename CT, typename R, int TC>
+template <typename CT, typename R, int TC, bool GATED>
 __global__ void __launch_bounds__(128) k_dense(const CT* __restrict__ a, int64_t m, int64_t n,
                                                const CT* __restrict__ x, int64_t xes, int64_t xcs,
                                                CT* __restrict__ y, int64_t yes, int64_t ycs, int64_t ncols,
                                                int64_t kc, CT* __restrict__ part, double ar, double ai,
-                                               double br, double bi) {
+                                               double br, double bi, FmaGate gate) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t c0 = (int64_t)blockIdx.y * TC;
+  if (GATED && !gate_open(gate, c0)) return;  // its tiles are multiples of TC vectors
   if (i >= m) return;
   const int nt = (int)(ncols - c0 < TC ? ncols - c0 : TC);
   const int64_t k0 = (int64_t)blockIdx.z * kc, k1 = k0 + kc < n ? k0 + kc : n;
@@ -149,14 +170,15 @@ __device__ __forceinline__ void combine64(double2* yp, double2 v, double ar, dou
   *yp = make_double2(re, im);
 }
 
-template <int TC>
+template <int TC, bool GATED>
 __global__ void __launch_bounds__(128) k_dense_ff(const float4* __restrict__ a, int64_t m, int64_t n,
                                                   const float4* __restrict__ x, int64_t xes, int64_t xcs,
                                                   double2* __restrict__ y, int64_t yes, int64_t ycs, int64_t ncols,
                                                   int64_t kc, double2* __restrict__ part, double ar, double ai,
-                                                  double br, double bi) {
+                                                  double br, double bi, FmaGate gate) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t c0 = (int64_t)blockIdx.y * TC;
+  if (GATED && !gate_open(gate, c0)) return;
   if (i >= m) return;
   const int nt = (int)(ncols - c0 < TC ? ncols - c0 : TC);
   const int64_t k0 = (int64_t)blockIdx.z * kc, k1 = k0 + kc < n ? k0 + kc : n;
@@ -182,30 +204,36 @@ __global__ void __launch_bounds__(128) k_dense_ff(const float4* __restrict__ a, 
   }
 }
 
+template <bool GATED>
 __global__ void k_modek_ff(const float4* __restrict__ A, int64_t s1, int64_t dout, int64_t din, int64_t s3,
                            const float4* __restrict__ x, int64_t xes, int64_t xcs, double2* __restrict__ y,
-                           int64_t yes, int64_t ycs, int64_t ncols, double ar, double ai, double br, double bi) {
+                           int64_t yes, int64_t ycs, int64_t ncols, double ar, double ai, double br, double bi,
+                           FmaGate gate) {
   const int64_t len = s1 * dout * s3;
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t c = blockIdx.y;
-  if (i >= len || c >= ncols) return;
-  int64_t a, t, j, b;
-  udivmod(i, s1, t, a);
-  udivmod(t, dout, b, j);
-  const float4* xc = x + c * xcs;
-  gather::AccFF acc;
-  acc.zero();
-  for (int64_t k = 0; k < din; ++k) acc.mac(A[j + k * dout], xc[(a + s1 * (k + din * b)) * xes]);
-  combine64(y + i * yes + c * ycs, ff_total(acc), ar, ai, br, bi);
+  if (c >= ncols) return;
+  auto element = [&](int64_t i) {
+    int64_t a, t, j, b;
+    udivmod(i, s1, t, a);
+    udivmod(t, dout, b, j);
+    if (GATED && !left_to_fma(gate, a + s1 * (b + s3 * (gate.c0 + c)))) return;
+    const float4* xc = x + c * xcs;
+    gather::AccFF acc;
+    acc.zero();
+    for (int64_t k = 0; k < din; ++k) acc.mac(A[j + k * dout], xc[(a + s1 * (k + din * b)) * xes]);
+    combine64(y + i * yes + c * ycs, ff_total(acc), ar, ai, br, bi);
+  };
+  each_element<GATED>(len, gate, element);
 }
 
 // The k ranges' partial sums of k_dense added in order, then alpha / beta.
-template <typename CT, typename R>
+template <typename CT, typename R, bool GATED>
 __global__ void k_dense_reduce(const CT* __restrict__ part, int kchunks, int64_t m, int64_t ncols,
                                CT* __restrict__ y, int64_t yes, int64_t ycs, double ar, double ai, double br,
-                               double bi) {
+                               double bi, FmaGate gate) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t c = blockIdx.y;
+  if (GATED && !gate_open(gate, c)) return;
   if (i >= m) return;
   R sre = 0, sim = 0;
   for (int z = 0; z < kchunks; ++z) {
@@ -227,45 +255,48 @@ __global__ void k_dense_reduce(const CT* __restrict__ part, int kchunks, int64_t
 // One mode product: out[a, j, b] = alpha * sum_k A[j, k] in[a, k, b] + beta * out,
 // a < s1, j < dout, b < s3; element e of vector c at x[e * xes + c * xcs].
 // A non-square Eye is the truncated identity (src/operators_lazytensor.jl:348-371).
-template <typename CT, typename R, bool EYE>
+template <typename CT, typename R, bool EYE, bool GATED>
 __global__ void k_modek(const CT* __restrict__ A, int64_t s1, int64_t dout, int64_t din, int64_t s3,
                         const CT* __restrict__ x, int64_t xes, int64_t xcs, CT* __restrict__ y,
                         int64_t yes, int64_t ycs, int64_t ncols, double ar, double ai, double br,
-                        double bi) {
+                        double bi, FmaGate gate) {
   const int64_t len = s1 * dout * s3;
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t c = blockIdx.y;
-  if (i >= len || c >= ncols) return;
-  int64_t a, t, j, b;
-  udivmod(i, s1, t, a);
-  udivmod(t, dout, b, j);
-  const CT* xc = x + c * xcs;
-  R sre = 0, sim = 0;
-  if (EYE) {
-    if (j < din) {
-      CT xv = xc[(a + s1 * (j + din * b)) * xes];
-      sre = xv.x;
-      sim = xv.y;
+  if (c >= ncols) return;
+  auto element = [&](int64_t i) {
+    int64_t a, t, j, b;
+    udivmod(i, s1, t, a);
+    udivmod(t, dout, b, j);
+    if (GATED && !left_to_fma(gate, a + s1 * (b + s3 * (gate.c0 + c)))) return;
+    const CT* xc = x + c * xcs;
+    R sre = 0, sim = 0;
+    if (EYE) {
+      if (j < din) {
+        CT xv = xc[(a + s1 * (j + din * b)) * xes];
+        sre = xv.x;
+        sim = xv.y;
+      }
+    } else {
+      for (int64_t k = 0; k < din; ++k) {
+        CT av = A[j + k * dout];
+        CT xv = xc[(a + s1 * (k + din * b)) * xes];
+        sre = fma(av.x, xv.x, sre);
+        sre = fma(-av.y, xv.y, sre);
+        sim = fma(av.x, xv.y, sim);
+        sim = fma(av.y, xv.x, sim);
+      }
     }
-  } else {
-    for (int64_t k = 0; k < din; ++k) {
-      CT av = A[j + k * dout];
-      CT xv = xc[(a + s1 * (k + din * b)) * xes];
-      sre = fma(av.x, xv.x, sre);
-      sre = fma(-av.y, xv.y, sre);
-      sim = fma(av.x, xv.y, sim);
-      sim = fma(av.y, xv.x, sim);
+    R re = (R)ar * sre - (R)ai * sim;
+    R im = (R)ar * sim + (R)ai * sre;
+    CT* yp = y + i * yes + c * ycs;
+    if (br != 0.0 || bi != 0.0) {
+      CT o = *yp;
+      re += (R)br * o.x - (R)bi * o.y;
+      im += (R)br * o.y + (R)bi * o.x;
     }
-  }
-  R re = (R)ar * sre - (R)ai * sim;
-  R im = (R)ar * sim + (R)ai * sre;
-  CT* yp = y + i * yes + c * ycs;
-  if (br != 0.0 || bi != 0.0) {
-    CT o = *yp;
-    re += (R)br * o.x - (R)bi * o.y;
-    im += (R)br * o.y + (R)bi * o.x;
-  }
-  *yp = mk<CT>(re, im);
+    *yp = mk<CT>(re, im);
+  };
+  each_element<GATED>(len, gate, element);
 }
 
 // ---------------------------------------------------------------------------
@@ -391,7 +422,7 @@ int dense_kchunks(int64_t m, int64_t n, int64_t ncols, int tc) {
 template <typename CT, typename R>
 void dense_typed(const void* a, int64_t m, int64_t n, c128 alpha, const void* x, int64_t xes, int64_t xcs,
                  c128 beta, void* y, int64_t yes, int64_t ycs, int64_t ncols, Workspace* ws, int slot,
-                 cudaStream_t s) {
+                 cudaStream_t s, const FmaGate& gate) {
   const int tc = ncols >= 8 ? 8 : ncols >= 4 ? 4 : ncols >= 2 ? 2 : 1;
   int kch = ws ? dense_kchunks(m, n, ncols, tc) : 1;
   CT* part = nullptr;
@@ -399,36 +430,28 @@ void dense_typed(const void* a, int64_t m, int64_t n, c128 alpha, const void* x,
   const int64_t kc = (n + kch - 1) / kch;
   kch = (int)((n + kc - 1) / kc);
   const dim3 grid(blocks_for(m, 128), (unsigned)((ncols + tc - 1) / tc), (unsigned)kch);
-  const CT* A = (const CT*)a;
-  const CT* X = (const CT*)x;
-  CT* Y = (CT*)y;
+  const bool gated = gate.any != nullptr;
+  auto run = [&](auto kern) {
+    launch_kernel(gated, kern, grid, 128u, 0, s, (const CT*)a, m, n, (const CT*)x, xes, xcs, (CT*)y, yes, ycs, ncols, kc,
+                  part, alpha.re, alpha.im, beta.re, beta.im, gate);
+    QOB_LAUNCHED();
+  };
   switch (tc) {
-    case 8:
-      k_dense<CT, R, 8><<<grid, 128, 0, s>>>(A, m, n, X, xes, xcs, Y, yes, ycs, ncols, kc, part, alpha.re,
-                                             alpha.im, beta.re, beta.im);
-      break;
-    case 4:
-      k_dense<CT, R, 4><<<grid, 128, 0, s>>>(A, m, n, X, xes, xcs, Y, yes, ycs, ncols, kc, part, alpha.re,
-                                             alpha.im, beta.re, beta.im);
-      break;
-    case 2:
-      k_dense<CT, R, 2><<<grid, 128, 0, s>>>(A, m, n, X, xes, xcs, Y, yes, ycs, ncols, kc, part, alpha.re,
-                                             alpha.im, beta.re, beta.im);
-      break;
-    default:
-      k_dense<CT, R, 1><<<grid, 128, 0, s>>>(A, m, n, X, xes, xcs, Y, yes, ycs, ncols, kc, part, alpha.re,
-                                             alpha.im, beta.re, beta.im);
+    case 8: run(gated ? k_dense<CT, R, 8, true> : k_dense<CT, R, 8, false>); break;
+    case 4: run(gated ? k_dense<CT, R, 4, true> : k_dense<CT, R, 4, false>); break;
+    case 2: run(gated ? k_dense<CT, R, 2, true> : k_dense<CT, R, 2, false>); break;
+    default: run(k_dense<CT, R, 1, false>);  // a gate comes with two vectors and more
   }
-  QOB_LAUNCHED();
   if (part) {
-    k_dense_reduce<CT, R><<<dim3(blocks_for(m, 128), (unsigned)ncols), 128, 0, s>>>(
-        part, kch, m, ncols, Y, yes, ycs, alpha.re, alpha.im, beta.re, beta.im);
+    launch_kernel(gated, gated ? k_dense_reduce<CT, R, true> : k_dense_reduce<CT, R, false>,
+                  dim3(blocks_for(m, 128), (unsigned)ncols), 128u, 0, s, (const CT*)part, kch, m, ncols, (CT*)y, yes, ycs,
+                  alpha.re, alpha.im, beta.re, beta.im, gate);
     QOB_LAUNCHED();
   }
 }
 void dense_ff(const void* a, int64_t m, int64_t n, c128 alpha, const void* x, int64_t xes, int64_t xcs,
               c128 beta, void* y, int64_t yes, int64_t ycs, int64_t ncols, Workspace* ws, int slot,
-              cudaStream_t s) {
+              cudaStream_t s, const FmaGate& gate) {
   const int tc = ncols >= 4 ? 4 : ncols >= 2 ? 2 : 1;
   int kch = ws ? dense_kchunks(m, n, ncols, tc) : 1;
   double2* part = nullptr;
@@ -436,26 +459,21 @@ void dense_ff(const void* a, int64_t m, int64_t n, c128 alpha, const void* x, in
   const int64_t kc = (n + kch - 1) / kch;
   kch = (int)((n + kc - 1) / kc);
   const dim3 grid(blocks_for(m, 128), (unsigned)((ncols + tc - 1) / tc), (unsigned)kch);
-  const float4* A = (const float4*)a;
-  const float4* X = (const float4*)x;
-  double2* Y = (double2*)y;
+  const bool gated = gate.any != nullptr;
+  auto run = [&](auto kern) {
+    launch_kernel(gated, kern, grid, 128u, 0, s, (const float4*)a, m, n, (const float4*)x, xes, xcs, (double2*)y, yes, ycs,
+                  ncols, kc, part, alpha.re, alpha.im, beta.re, beta.im, gate);
+    QOB_LAUNCHED();
+  };
   switch (tc) {
-    case 4:
-      k_dense_ff<4><<<grid, 128, 0, s>>>(A, m, n, X, xes, xcs, Y, yes, ycs, ncols, kc, part, alpha.re, alpha.im,
-                                         beta.re, beta.im);
-      break;
-    case 2:
-      k_dense_ff<2><<<grid, 128, 0, s>>>(A, m, n, X, xes, xcs, Y, yes, ycs, ncols, kc, part, alpha.re, alpha.im,
-                                         beta.re, beta.im);
-      break;
-    default:
-      k_dense_ff<1><<<grid, 128, 0, s>>>(A, m, n, X, xes, xcs, Y, yes, ycs, ncols, kc, part, alpha.re, alpha.im,
-                                         beta.re, beta.im);
+    case 4: run(gated ? k_dense_ff<4, true> : k_dense_ff<4, false>); break;
+    case 2: run(gated ? k_dense_ff<2, true> : k_dense_ff<2, false>); break;
+    default: run(k_dense_ff<1, false>);
   }
-  QOB_LAUNCHED();
   if (part) {
-    k_dense_reduce<double2, double><<<dim3(blocks_for(m, 128), (unsigned)ncols), 128, 0, s>>>(
-        part, kch, m, ncols, Y, yes, ycs, alpha.re, alpha.im, beta.re, beta.im);
+    launch_kernel(gated, gated ? k_dense_reduce<double2, double, true> : k_dense_reduce<double2, double, false>,
+                  dim3(blocks_for(m, 128), (unsigned)ncols), 128u, 0, s, (const double2*)part, kch, m, ncols, (double2*)y,
+                  yes, ycs, alpha.re, alpha.im, beta.re, beta.im, gate);
     QOB_LAUNCHED();
   }
 }
@@ -463,14 +481,16 @@ void dense_ff(const void* a, int64_t m, int64_t n, c128 alpha, const void* x, in
 
 void launch_dense(int precision, const void* a, int64_t m, int64_t n, c128 alpha, const void* x,
                   int64_t xes, int64_t xcs, c128 beta, void* y, int64_t yes, int64_t ycs,
-                  int64_t ncols, cudaStream_t s, Workspace* ws, int slot, bool ff, bool dmma) {
+                  int64_t ncols, cudaStream_t s, Workspace* ws, int slot, bool ff, bool dmma, FmaGate gate) {
   if (m == 0 || ncols == 0) return;
   const size_t esz = precision == QOB_C128 ? 16 : 8;
   if (ncols > 65535 * 8) {  // grid.y limit: split the vectors
-    for (int64_t c0 = 0; c0 < ncols; c0 += 65535 * 8)
+    for (int64_t c0 = 0; c0 < ncols; c0 += 65535 * 8) {
       launch_dense(precision, a, m, n, alpha, (const char*)x + c0 * xcs * esz, xes, xcs, beta,
                    (char*)y + c0 * ycs * esz, yes, ycs, std::min<int64_t>(65535 * 8, ncols - c0), s, ws, slot,
-                   ff, dmma);
+                   ff, dmma, gate);
+      gate.c0 += 65535 * 8;
+    }
     return;
   }
   if (dmma && !ff && precision == QOB_C128 && n >= kDmmaMinK && ncols >= kDmmaMinCols) {
@@ -478,16 +498,17 @@ void launch_dense(int precision, const void* a, int64_t m, int64_t n, c128 alpha
     return;
   }
   if (ff)
-    dense_ff(a, m, n, alpha, x, xes, xcs, beta, y, yes, ycs, ncols, ws, slot, s);
+    dense_ff(a, m, n, alpha, x, xes, xcs, beta, y, yes, ycs, ncols, ws, slot, s, gate);
   else if (precision == QOB_C128)
-    dense_typed<double2, double>(a, m, n, alpha, x, xes, xcs, beta, y, yes, ycs, ncols, ws, slot, s);
+    dense_typed<double2, double>(a, m, n, alpha, x, xes, xcs, beta, y, yes, ycs, ncols, ws, slot, s, gate);
   else
-    dense_typed<float2, float>(a, m, n, alpha, x, xes, xcs, beta, y, yes, ycs, ncols, ws, slot, s);
+    dense_typed<float2, float>(a, m, n, alpha, x, xes, xcs, beta, y, yes, ycs, ncols, ws, slot, s, gate);
 }
 
 void launch_modek(int precision, const void* a, bool eye, int64_t s1, int64_t dout, int64_t din,
                   int64_t s3, c128 alpha, const void* x, int64_t xes, int64_t xcs, c128 beta,
-                  void* y, int64_t yes, int64_t ycs, int64_t ncols, cudaStream_t s, bool ff, bool dmma) {
+                  void* y, int64_t yes, int64_t ycs, int64_t ncols, cudaStream_t s, bool ff, bool dmma,
+                  FmaGate gate) {
   const int64_t len = s1 * dout * s3;
   if (len == 0 || ncols == 0) return;
   if (dmma && !ff && !eye && precision == QOB_C128 && din >= kDmmaMinK && ncols >= kDmmaMinCols) {
@@ -496,33 +517,37 @@ void launch_modek(int precision, const void* a, bool eye, int64_t s1, int64_t do
   }
   const size_t esz = precision == QOB_C128 ? 16 : 8;
   if (ncols > 65535) {  // grid.y limit: split the vectors
-    for (int64_t c0 = 0; c0 < ncols; c0 += 65535)
+    for (int64_t c0 = 0; c0 < ncols; c0 += 65535) {
       launch_modek(precision, a, eye, s1, dout, din, s3, alpha, (const char*)x + c0 * xcs * esz, xes, xcs,
-                   beta, (char*)y + c0 * ycs * esz, yes, ycs, std::min<int64_t>(65535, ncols - c0), s, ff, dmma);
+                   beta, (char*)y + c0 * ycs * esz, yes, ycs, std::min<int64_t>(65535, ncols - c0), s, ff, dmma, gate);
+      gate.c0 += 65535;
+    }
     return;
   }
-  dim3 grid(blocks_for(len, 256), (unsigned)ncols);
+  const bool gated = gate.any != nullptr;
+  unsigned blocks = blocks_for(len, 256);
+  if (gated) {  // most often there is nothing to do: 16 blocks an SM at most (8 leave graded kets a ragged wave)
+    const unsigned most = (unsigned)((16 * (int64_t)gather::current_sms() + ncols - 1) / ncols);
+    blocks = std::min(blocks, most);
+  }
+  auto run = [&](auto kern, auto* A, auto* X, auto* Y) {
+    launch_kernel(gated, kern, dim3(blocks, (unsigned)ncols), 256u, 0, s, A, s1, dout, din, s3, X, xes, xcs, Y, yes, ycs,
+                  ncols, alpha.re, alpha.im, beta.re, beta.im, gate);
+  };
   if (ff && !eye) {
-    k_modek_ff<<<grid, 256, 0, s>>>((const float4*)a, s1, dout, din, s3, (const float4*)x, xes, xcs, (double2*)y,
-                                    yes, ycs, ncols, alpha.re, alpha.im, beta.re, beta.im);
+    run(gated ? k_modek_ff<true> : k_modek_ff<false>, (const float4*)a, (const float4*)x, (double2*)y);
   } else if (precision == QOB_C128) {
     if (eye)
-      k_modek<double2, double, true><<<grid, 256, 0, s>>>(nullptr, s1, dout, din, s3, (const double2*)x, xes,
-                                                          xcs, (double2*)y, yes, ycs, ncols, alpha.re,
-                                                          alpha.im, beta.re, beta.im);
+      run(k_modek<double2, double, true, false>, (const double2*)nullptr, (const double2*)x, (double2*)y);
     else
-      k_modek<double2, double, false><<<grid, 256, 0, s>>>((const double2*)a, s1, dout, din, s3,
-                                                           (const double2*)x, xes, xcs, (double2*)y, yes,
-                                                           ycs, ncols, alpha.re, alpha.im, beta.re, beta.im);
+      run(gated ? k_modek<double2, double, false, true> : k_modek<double2, double, false, false>, (const double2*)a,
+          (const double2*)x, (double2*)y);
   } else {
     if (eye)
-      k_modek<float2, float, true><<<grid, 256, 0, s>>>(nullptr, s1, dout, din, s3, (const float2*)x, xes, xcs,
-                                                        (float2*)y, yes, ycs, ncols, alpha.re, alpha.im,
-                                                        beta.re, beta.im);
+      run(k_modek<float2, float, true, false>, (const float2*)nullptr, (const float2*)x, (float2*)y);
     else
-      k_modek<float2, float, false><<<grid, 256, 0, s>>>((const float2*)a, s1, dout, din, s3,
-                                                         (const float2*)x, xes, xcs, (float2*)y, yes, ycs,
-                                                         ncols, alpha.re, alpha.im, beta.re, beta.im);
+      run(gated ? k_modek<float2, float, false, true> : k_modek<float2, float, false, false>, (const float2*)a,
+          (const float2*)x, (float2*)y);
   }
   QOB_LAUNCHED();
 }

@@ -26,8 +26,8 @@
 // for every row, vector and chunk, Re and Im apart: no more than the bound of a chain of
 // multiply-adds over 4 terms, and the counts ask for more.  A tile of vectors that fails (graded
 // ones, sparse ones, components that are not finite or far from 1) is left
-// to the FMA arithmetic of the form: the split kernel flags it, the GEMM does not
-// store it and k_slice_fallback computes it.  A matrix that fails with vectors of ones has no
+// to the FMA kernels: the split kernel flags it, the GEMM does not store it and the
+// FMA kernels, launched behind it, compute the flagged tiles alone (FmaGate).  A matrix that fails with vectors of ones has no
 // planes.  Gaussian entries (matrices of 32 to 4096 rows) reach 0.2 of the limit in ComplexF32
 // and double-float and 0.7 in ComplexF64, and 650 of the 1024 that keep a diagonal exact.
 //
@@ -274,8 +274,8 @@ template <int FORM, int ROWS, bool INTER, typename IN>
 __global__ void __launch_bounds__(split_threads(ROWS)) k_slice_split(const IN* __restrict__ x, int64_t n, int64_t es, TcColMap map,
                                                      int64_t nvec, int nkb, int kfast, int sub,
                                                      unsigned char* __restrict__ out, int* __restrict__ exps,
-                                                     int* __restrict__ flags, const SliceSide* __restrict__ other,
-                                                     SliceSide* __restrict__ own) {
+                                                     int* __restrict__ flags, int* __restrict__ any,
+                                                     const SliceSide* __restrict__ other, SliceSide* __restrict__ own) {
   constexpr int S = Sl<FORM>::S, H = ROWS / 2, kSlSplit = split_threads(ROWS);
   using C2 = decltype(as_value(IN{}));
   using T = decltype(C2{}.x);
@@ -294,6 +294,7 @@ __global__ void __launch_bounds__(split_threads(ROWS)) k_slice_split(const IN* _
   C2* t = reinterpret_cast<C2*>(sl_smem);  // [vector][k]
   const int64_t v0 = (int64_t)blockIdx.x * H;
   if (threadIdx.x == 0) bad = worst1 = worst2 = 0;
+  if (any && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) *any = 0;  // set by the GEMM
   if (threadIdx.x < kLevels) side.c[threadIdx.x] = kSlChunk * 16;
   if (threadIdx.x < ROWS) cnt_hi[threadIdx.x] = cnt_lo[threadIdx.x] = sum1[threadIdx.x] = sum2[threadIdx.x] = 0u;
   if (threadIdx.x < H) off[threadIdx.x] = v0 + threadIdx.x < nvec ? col_offset(map, v0 + threadIdx.x) : -1;
@@ -534,7 +535,7 @@ struct SlAcc<QOB_C64> {
 template <int FORM, int BN>
 __global__ void __launch_bounds__(SlCfg<FORM, BN>::kThreads, 1)
     k_slice_gemm(const unsigned char* __restrict__ A, const int* __restrict__ ea, const unsigned char* __restrict__ B,
-                 const int* __restrict__ ex, const int* __restrict__ flags, int64_t m, int mt, int64_t ncols, int nkb,
+                 const int* __restrict__ ex, const int* __restrict__ flags, int* __restrict__ any, int* __restrict__ left, int64_t m, int mt, int64_t ncols, int nkb,
                  int nch, int per, int64_t units, int smax, int swap, typename Sl<FORM>::V* y, int64_t yes, TcColMap ym,
                  typename Sl<FORM>::V alpha, typename Sl<FORM>::V beta, typename Sl<FORM>::V* part, unsigned* status) {
   using C = SlCfg<FORM, BN>;
@@ -557,7 +558,7 @@ __global__ void __launch_bounds__(SlCfg<FORM, BN>::kThreads, 1)
   int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t u0 = (int64_t)blockIdx.x * per;
-  const int nu = (int)(units - u0 < (int64_t)per ? units - u0 : (int64_t)per);
+  int nu = (int)(units - u0 < (int64_t)per ? units - u0 : (int64_t)per);
   const int ch_start = (int)(u0 % nch);
   auto steps = [&](int ch) { return chunk_start(ch + 1, nkb, nch) - chunk_start(ch, nkb, nch); };
 
@@ -591,7 +592,19 @@ __global__ void __launch_bounds__(SlCfg<FORM, BN>::kThreads, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  pdl_enter();
+  pdl_wait();
+  {  // the tiles left to the FMA kernels; a run of nothing else is not done
+    bool live = false;
+    for (int64_t rt = u0 / nch + threadIdx.x; rt <= (u0 + nu - 1) / nch; rt += blockDim.x) {
+      const int64_t vt = swap ? rt % mt : rt / mt;
+      int f = 0;
+      for (int j = 0; j < nch; ++j) f |= flags[vt * nch + j];
+      left[vt] = f;  // by each of its blocks
+      if (f) *any = 1;
+      live |= f == 0;
+    }
+    if (!__syncthreads_or(live)) nu = 0;
+  }
 
   // warps 1 and 2 meet; true when either asks to stop
   auto meet = [&](bool ask) {
@@ -877,12 +890,12 @@ __device__ __forceinline__ void axpby_out(V* yp, T re, T im, V alpha, V beta) {
 
 // y of the row tiles split over several blocks: their partial products in chunk order
 template <int FORM, int BN>
-__global__ void k_slice_reduce(const typename Sl<FORM>::V* __restrict__ part, const int* __restrict__ flags, int mt,
+__global__ void k_slice_reduce(const typename Sl<FORM>::V* __restrict__ part, const int* __restrict__ left, int mt,
                                int nch, int per, int smax, int swap, int64_t m, int64_t ncols,
                                typename Sl<FORM>::V* y, int64_t yes, TcColMap ym, typename Sl<FORM>::V alpha, typename Sl<FORM>::V beta) {
   using T = typename SlAcc<FORM>::T;
   constexpr int H = BN / 2;
-  pdl_enter();
+  pdl_wait();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= m) return;
   const int il = (int)(i % (kSlRows / 2));
@@ -891,9 +904,7 @@ __global__ void k_slice_reduce(const typename Sl<FORM>::V* __restrict__ part, co
     const int64_t ct = cg / H, rt = ct * mt + mti;
     const int64_t b0 = rt * nch / per, b1 = (rt * nch + nch - 1) / per;
     if (b0 == b1) continue;  // one block wrote it
-    bool skip = false;
-    for (int j = 0; j < nch; ++j) skip |= flags[(swap ? mti : ct) * nch + j] != 0;
-    if (skip) continue;
+    if (left[swap ? mti : ct]) continue;
     T re = 0, im = 0;
     for (int64_t j = 0; j <= b1 - b0; ++j) {
       const typename Sl<FORM>::V p = part[((rt * smax + j) * H + cg % H) * (kSlRows / 2) + il];
@@ -904,49 +915,10 @@ __global__ void k_slice_reduce(const typename Sl<FORM>::V* __restrict__ part, co
   }
 }
 
-// The flagged column tiles in the form's FMA arithmetic: a thread per row, the
-// tile's vectors one after another.
-template <int FORM>
-__global__ void __launch_bounds__(128) k_slice_fallback(const typename Sl<FORM>::M* __restrict__ a, int64_t m, int64_t n,
-                                                        const typename Sl<FORM>::V* __restrict__ x, int64_t es,
-                                                        TcColMap xm, const int* __restrict__ flags, int nch,
-                                                        int64_t tile, int64_t ncols, typename Sl<FORM>::V* y, int64_t yes,
-                                                        TcColMap ym, typename Sl<FORM>::V alpha,
-                                                        typename Sl<FORM>::V beta) {
-  pdl_enter();
-  const int64_t ct = blockIdx.x;
-  bool run = false;
-  for (int j = 0; j < nch; ++j) run |= flags[ct * nch + j] != 0;
-  if (!run) return;
-  const int64_t i = blockIdx.y * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  for (int64_t c = ct * tile; c < ncols && c < (ct + 1) * tile; ++c) {
-    const typename Sl<FORM>::V* xc = x + col_offset(xm, c);
-    auto* yp = y + i * yes + col_offset(ym, c);
-    if constexpr (FORM == QOB_C128X) {
-      gather::AccFF acc;
-      acc.zero();
-      for (int64_t k = 0; k < n; ++k) acc.mac(a[i + k * m], gather::ff_split4(xc[k * es]));
-      axpby_out(yp, gather::ff_join(acc.rh, acc.rl), gather::ff_join(acc.ih, acc.il), alpha, beta);
-    } else {
-      using T = typename SlAcc<FORM>::T;
-      T re = 0, im = 0;
-      for (int64_t k = 0; k < n; ++k) {
-        const typename Sl<FORM>::V av = a[i + k * m], xv = xc[k * es];
-        re = fma(av.x, xv.x, re);
-        re = fma(-av.y, xv.y, re);
-        im = fma(av.x, xv.y, im);
-        im = fma(av.y, xv.x, im);
-      }
-      axpby_out(yp, re, im, alpha, beta);
-    }
-  }
-}
-
 template <int FORM, int ROWS, bool INTER, typename IN>
 void run_split(const IN* x, int64_t n, int64_t es, const TcColMap& map, int64_t nvec, int64_t tiles, int nkb,
-               unsigned char* out, int* exps, int* flags, const SliceSide* other, SliceSide* own, cudaStream_t s,
-               bool pdl) {
+               unsigned char* out, int* exps, int* flags, int* any, const SliceSide* other, SliceSide* own,
+               cudaStream_t s, bool pdl) {
   const int nch = (nkb + kSlChunk - 1) / kSlChunk;
   auto kern = k_slice_split<FORM, ROWS, INTER, IN>;
   // k steps staged at a time: the chunk where it fits beside the tile's tables, otherwise half
@@ -957,15 +929,15 @@ void run_split(const IN* x, int64_t n, int64_t es, const TcColMap& map, int64_t 
   const size_t smem = bytes(sub);
   QOB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   launch_kernel(pdl, kern, dim3((unsigned)tiles, (unsigned)nch), (unsigned)split_threads(ROWS), smem, s, x, n, es, map, nvec, nkb,
-                es == 1 ? 1 : 0, sub, out, exps, flags, other, own);
+                es == 1 ? 1 : 0, sub, out, exps, flags, any, other, own);
   QOB_LAUNCHED();
 }
 
 // swap: the vectors are the M side (their bytes widened), the matrix the N side.
 template <int FORM, int BN>
-void run_slices(const SliceDense& d, bool swap, const void* a, const void* xv, int64_t xes, const TcColMap& xm,
-                int64_t ncols, void* yv, int64_t yes, const TcColMap& ym, c128 al, c128 be, Workspace* ws, int slot,
-                cudaStream_t s, unsigned* status, int num_sms, bool pdl) {
+FmaGate run_slices(const SliceDense& d, bool swap, const void* xv, int64_t xes, const TcColMap& xm, int64_t ncols, void* yv,
+                   int64_t yes, const TcColMap& ym, c128 al, c128 be, Workspace* ws, int slot, cudaStream_t s,
+                   unsigned* status, int num_sms, bool pdl) {
   using C = SlCfg<FORM, BN>;
   using V = typename Sl<FORM>::V;
   using T = typename SlAcc<FORM>::T;
@@ -989,37 +961,41 @@ void run_slices(const SliceDense& d, bool swap, const void* a, const void* xv, i
   const int64_t tile = swap ? HM : H;  // vectors of a tile
   const SlicePlanes& pl = swap ? d.nside : d.mside;
   const SliceSide* sides = static_cast<const SliceSide*>(pl.sides.p);
-  const size_t bbytes = (size_t)vt * nkb * (swap ? C::kA : C::kB), ebytes = (size_t)vt * nch * (tile + 1) * sizeof(int);
+  const size_t bbytes = (size_t)vt * nkb * (swap ? C::kA : C::kB), ebytes = ((size_t)vt * (nch * (tile + 1) + 1) + 1) * sizeof(int);
   unsigned char* w = static_cast<unsigned char*>(ws->get(slot, bbytes + ebytes));
   int* exps = reinterpret_cast<int*>(w + bbytes);
   int* flags = exps + vt * nch * tile;
+  int *left = flags + vt * nch, *any = left + vt;
   V* part = nullptr;
   if (per % nch != 0) part = static_cast<V*>(ws->get(slot + 1, (size_t)rtiles * smax * H * HM * sizeof(V)));
   if (swap)
-    run_split<FORM, kSlRows, true, V>(x, d.n, xes, xm, ncols, vt, nkb, w, exps, flags, sides, nullptr, s, pdl);
+    run_split<FORM, kSlRows, true, V>(x, d.n, xes, xm, ncols, vt, nkb, w, exps, flags, any, sides, nullptr, s, pdl);
   else
-    run_split<FORM, BN, false, V>(x, d.n, xes, xm, ncols, vt, nkb, w, exps, flags, sides, nullptr, s, pdl);
+    run_split<FORM, BN, false, V>(x, d.n, xes, xm, ncols, vt, nkb, w, exps, flags, any, sides, nullptr, s, pdl);
   const unsigned char* mp = swap ? w : static_cast<const unsigned char*>(pl.planes.p);
   const unsigned char* np = swap ? static_cast<const unsigned char*>(pl.planes.p) : w;
   const int* me = swap ? exps : static_cast<const int*>(pl.exps.p);
   const int* ne = swap ? static_cast<const int*>(pl.exps.p) : exps;
   auto kern = k_slice_gemm<FORM, BN>;
   QOB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem));
-  launch_kernel(pdl, kern, dim3((unsigned)blocks), (unsigned)C::kThreads, C::smem, s, mp, me, np, ne, (const int*)flags,
-                mrows, (int)mt, nrows, nkb, nch, (int)per, units, smax, swap ? 1 : 0, y, yes, ym, alpha, beta, part,
+  // the launches behind the split kernel overlap with the one before (pdl_enter, pdl_wait): the
+  // GEMM's blocks set themselves up beside the split's (4096 x 4096 on 16 kets, ComplexF32, 89 -> 83 us)
+  launch_kernel(true, kern, dim3((unsigned)blocks), (unsigned)C::kThreads, C::smem, s, mp, me, np, ne, (const int*)flags,
+                any, left, mrows, (int)mt, nrows, nkb, nch, (int)per, units, smax, swap ? 1 : 0, y, yes, ym, alpha, beta, part,
                 status);
   QOB_LAUNCHED();
   if (part) {
-    launch_kernel(pdl, k_slice_reduce<FORM, BN>,
+    launch_kernel(true, k_slice_reduce<FORM, BN>,
                   dim3((unsigned)((mrows + 127) / 128), (unsigned)std::min<int64_t>(nrows, 65535)), 128u, 0, s,
-                  (const V*)part, (const int*)flags, (int)mt, nch, (int)per, smax, swap ? 1 : 0, mrows, nrows, y, yes,
+                  (const V*)part, (const int*)left, (int)mt, nch, (int)per, smax, swap ? 1 : 0, mrows, nrows, y, yes,
                   ym, alpha, beta);
     QOB_LAUNCHED();
   }
-  launch_kernel(pdl, k_slice_fallback<FORM>, dim3((unsigned)vt, (unsigned)((d.m + 127) / 128)), 128u, 0, s,
-                static_cast<const typename Sl<FORM>::M*>(a), d.m, d.n, x, xes, xm, (const int*)flags, nch, tile, ncols,
-                y, yes, ym, alpha, beta);
-  QOB_LAUNCHED();
+  FmaGate g;
+  g.any = any;
+  g.tiles = left;
+  while (((int64_t)1 << g.log2_tile) < tile) ++g.log2_tile;
+  return g;
 }
 
 constexpr int kSwapBN = 64;
@@ -1044,11 +1020,11 @@ void build_slices(SliceDense& d, bool swap, const void* a, cudaStream_t s) {
   if (swap)
     run_split<FORM, kSwapBN, false, typename Sl<FORM>::M>(m, d.n, d.m, map, d.m, tiles, d.nkb,
                                                           static_cast<unsigned char*>(pl.planes.p), exps, flags,
-                                                          nullptr, tile_sides, s, false);
+                                                          nullptr, nullptr, tile_sides, s, false);
   else
     run_split<FORM, kSlRows, true, typename Sl<FORM>::M>(m, d.n, d.m, map, d.m, tiles, d.nkb,
                                                          static_cast<unsigned char*>(pl.planes.p), exps, flags,
-                                                         nullptr, tile_sides, s, false);
+                                                         nullptr, nullptr, tile_sides, s, false);
   std::vector<int> f((size_t)(tiles * nch));
   std::vector<SliceSide> q((size_t)(tiles * nch)), worst((size_t)nch);
   QOB_CUDA(cudaMemcpyAsync(f.data(), flags, f.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1115,18 +1091,15 @@ bool slice_ready(SliceDense& d, int form, const void* a, int64_t m, int64_t n, b
   return pl.state > 0;
 }
 
-void launch_slices(const SliceDense& d, int form, const void* a, c128 alpha, const void* x, int64_t xes,
-                   const TcColMap& xm, c128 beta, void* y, int64_t yes, const TcColMap& ym, int64_t ncols,
-                   cudaStream_t s, Workspace* ws, int slot, unsigned* status, int num_sms, bool pdl) {
+FmaGate launch_slices(const SliceDense& d, int form, c128 alpha, const void* x, int64_t xes, const TcColMap& xm,
+                      c128 beta, void* y, int64_t yes, const TcColMap& ym, int64_t ncols, cudaStream_t s, Workspace* ws,
+                      int slot, unsigned* status, int num_sms, bool pdl) {
   const bool swap = slice_swap(yes, ym, ncols);
 #define QOB_SL(F, BN) \
-  run_slices<F, BN>(d, swap, a, x, xes, xm, ncols, y, yes, ym, alpha, beta, ws, slot, s, status, num_sms, pdl)
-  if (form == QOB_C128)
-    ncols <= 16 ? QOB_SL(QOB_C128, 32) : QOB_SL(QOB_C128, kSwapBN);
-  else if (form == QOB_C128X)
-    ncols <= 16 ? QOB_SL(QOB_C128X, 32) : QOB_SL(QOB_C128X, kSwapBN);
-  else
-    ncols <= 16 ? QOB_SL(QOB_C64, 32) : QOB_SL(QOB_C64, kSwapBN);
+  run_slices<F, BN>(d, swap, x, xes, xm, ncols, y, yes, ym, alpha, beta, ws, slot, s, status, num_sms, pdl)
+  if (form == QOB_C128) return ncols <= 16 ? QOB_SL(QOB_C128, 32) : QOB_SL(QOB_C128, kSwapBN);
+  if (form == QOB_C128X) return ncols <= 16 ? QOB_SL(QOB_C128X, 32) : QOB_SL(QOB_C128X, kSwapBN);
+  return ncols <= 16 ? QOB_SL(QOB_C64, 32) : QOB_SL(QOB_C64, kSwapBN);
 #undef QOB_SL
 }
 

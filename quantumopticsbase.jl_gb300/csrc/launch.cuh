@@ -23,6 +23,15 @@ __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// The same without the second part: the next such launch starts when this grid has ended,
+// its blocks spread over the SMs as an ordinary launch's.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Whether column c is one that the gate leaves to the FMA kernels.
+__device__ __forceinline__ bool left_to_fma(const FmaGate& g, int64_t c) {
+  return g.tiles[c >> g.log2_tile] != 0;
+}
+
 // A launch with the programmatic stream-serialization attribute when pdl is set
 // (the kernel calls pdl_enter before its first access to memory), else an
 // ordinary one.

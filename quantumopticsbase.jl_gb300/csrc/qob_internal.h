@@ -331,6 +331,16 @@ struct SliceDense {
   SlicePlanes mside, nside;
 };
 
+// The tiles of vectors that a product from digit planes left to the FMA kernels: 2^log2_tile
+// consecutive columns each, those whose entry of tiles is not zero; *any says whether there
+// is one.  Without `any` the FMA kernels compute every column.  They are launched behind the
+// product in any case.
+struct FmaGate {
+  const int *any = nullptr, *tiles = nullptr;
+  int log2_tile = 0;
+  int64_t c0 = 0;    // the first vector of the call in the whole product's
+};
+
 // Dense full-space term (GEMM / GEMV pass) or a mode-k sequence.
 struct DensePass {
   TermCoef coef;
@@ -484,7 +494,7 @@ void launch_scale(int precision, void* y, int64_t rows, int64_t cols, int64_t ld
 void launch_dense(int precision, const void* a, int64_t m, int64_t n, c128 alpha, const void* x,
                   int64_t xes, int64_t xcs, c128 beta, void* y, int64_t yes, int64_t ycs,
                   int64_t ncols, cudaStream_t s, Workspace* ws = nullptr, int slot = 0, bool ff = false,
-                  bool dmma = false);
+                  bool dmma = false, FmaGate gate = {});
 // The same on the FP64 tensor cores (k_dmma.cu; ComplexF64 only).
 void launch_dense_dmma(const void* a, int64_t m, int64_t n, c128 alpha, const void* x, int64_t xes, int64_t xcs,
                        c128 beta, void* y, int64_t yes, int64_t ycs, int64_t ncols, cudaStream_t s, Workspace* ws,
@@ -510,13 +520,14 @@ bool launch_gemm_tc(const TcDense& d, c128 alpha, const void* x, int64_t xes, co
 // QOB_C64 or QOB_C128X) from its digit planes (k_slice.cu): columns as
 // launch_gemm_tc's; x unsplit.  slice_swap: which side the vectors take; slice_ready
 // makes the matrix's planes for it if they are not there yet (not inside a capture)
-// and says whether they can be used.  Workspace slots slot, slot + 1.
+// and says whether they can be used.  Workspace slots slot, slot + 1.  The columns of
+// the tiles that the returned gate names are not written: the FMA kernels follow with it.
 constexpr int64_t kSliceMin = 32;  // rows and columns from which a matrix gets planes
 bool slice_swap(int64_t yes, const TcColMap& ym, int64_t ncols);
 bool slice_ready(SliceDense& d, int form, const void* a, int64_t m, int64_t n, bool swap, cudaStream_t s);
-void launch_slices(const SliceDense& d, int form, const void* a, c128 alpha, const void* x, int64_t xes,
-                   const TcColMap& xm, c128 beta, void* y, int64_t yes, const TcColMap& ym, int64_t ncols,
-                   cudaStream_t s, Workspace* ws, int slot, unsigned* status, int num_sms, bool pdl);
+FmaGate launch_slices(const SliceDense& d, int form, c128 alpha, const void* x, int64_t xes, const TcColMap& xm,
+                      c128 beta, void* y, int64_t yes, const TcColMap& ym, int64_t ncols, cudaStream_t s, Workspace* ws,
+                      int slot, unsigned* status, int num_sms, bool pdl);
 // contracted dimension and kets from which the FP64 tensor-core option
 // applies (an 8 x 8 x 4 tile covers 8 kets: on one ket the FMA kernels are
 // about 15x faster at n = 4096)
@@ -524,11 +535,13 @@ constexpr int64_t kDmmaMinK = 64;
 constexpr int64_t kDmmaMinCols = 8;
 // Split of ncols vectors of n ComplexF64 elements (element stride es, vector
 // stride cs) into double-float quadruples at the same offsets of out.
-void launch_ff_split(const void* x, int64_t n, int64_t ncols, int64_t es, int64_t cs, void* out, cudaStream_t s);
+// (nothing done where `any` is given and *any is zero)
+void launch_ff_split(const void* x, int64_t n, int64_t ncols, int64_t es, int64_t cs, void* out, cudaStream_t s,
+                     const int* any = nullptr);
 void launch_modek(int precision, const void* a, bool eye, int64_t s1, int64_t dout, int64_t din,
                   int64_t s3, c128 alpha, const void* x, int64_t xes, int64_t xcs, c128 beta,
                   void* y, int64_t yes, int64_t ycs, int64_t ncols, cudaStream_t s, bool ff = false,
-                  bool dmma = false);
+                  bool dmma = false, FmaGate gate = {});
 void launch_axpby(int precision, const void* x, int64_t xes, int64_t xcs, c128 alpha, void* y,
                   int64_t yes, int64_t ycs, c128 beta, int64_t len, int64_t ncols,
                   cudaStream_t s);

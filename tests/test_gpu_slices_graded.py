@@ -159,3 +159,70 @@ def test_graded_mode_products(side, form, tol, unit, u):
         assert rel_l2(got, ref) < tol, e
         if side == "left":  # rows 0 .. 3 of the first factor are the identity's
             assert rel_l2(got[:4], ref[:4]) < tol, e
+
+
+@pytest.mark.parametrize("form,tol,unit,u", FORMS)
+@pytest.mark.parametrize("side", ["left", "right"])
+def test_graded_kets_among_others(side, form, tol, unit, u):
+    """Some tiles of vectors from digits and some not, into a result that is accumulated."""
+    rng = Q.Rng(6)
+    n, k = 66 * 3 * 70, 60
+    bs = [Q.GenericBasis(d) for d in (66, 3, 70)]
+    b = Q.tensor_basis(*bs)
+    f = [_rounded(_matrix(rng, d, d), form) for d in (66, 70)]
+    modes = O.LazyTensor(b, b, (1, 3), (O.Operator(bs[0], bs[0], f[0]), O.Operator(bs[2], bs[2], f[1])))
+    A, B = (f[0], f[1]) if side == "left" else (f[0].T, f[1].T)
+    a = _rounded(_matrix(rng, 330, 330), form)
+    for op, dim, ref in (
+            (modes, n, lambda v: np.tensordot(np.tensordot(A, v.reshape(66, 3, 70, -1, order="F"), (1, 0)), B,
+                                              (2, 1)).transpose(0, 1, 3, 2).reshape(n, -1, order="F")),
+            (_dense(a), 330, lambda v: (a if side == "left" else a.T) @ v)):
+        cols = k if op is modes else 150
+        X, Y = rng.kets_data(dim, cols), rng.kets_data(dim, cols)
+        for c in (1, 40, cols - 1):
+            X[:, c] *= 2.0 ** -(30.0 * np.arange(dim) / dim)
+            X[::7, c] = 0.0
+        X, Y = _rounded(X, form), _rounded(Y, form)
+        want = (0.7 - 0.2j) * ref(X) + (0.3 - 0.1j) * Y
+        if side == "left":
+            got = _mul(op, X, Y, form, 0.3 - 0.1j)
+        else:
+            got = _mul(op, np.asfortranarray(X.T), np.asfortranarray(Y.T), form, 0.3 - 0.1j, side="right").T
+        assert rel_l2(got, want) < tol
+        for c in (0, 1, 40, cols - 1):
+            assert rel_l2(got[:, c], want[:, c]) < tol, c
+
+
+@pytest.mark.parametrize("form,tol,unit,u", FORMS)
+def test_graded_kets_cost_what_the_fma_kernels_do(form, tol, unit, u):
+    """The same kets under a matrix that has no planes (a graded one) go to the FMA kernels at once."""
+    import torch
+
+    from qobgpu.mul import mul_
+
+    n, k = 2048, 16
+    g = torch.Generator(device="cuda:0")
+    g.manual_seed(7)
+    dt = torch.complex64 if form == "c64" else torch.complex128
+    a = (torch.randn(n, n, dtype=torch.complex128, device="cuda:0", generator=g) / 45).to(dt).cpu().numpy().T
+    x = torch.randn(k, n, dtype=torch.complex128, device="cuda:0", generator=g)
+    x[:, 100:] *= 2.0 ** -30
+    y = torch.zeros(k, n, dtype=dt, device="cuda:0").t()
+    b, bk = Q.GenericBasis(n), Q.GenericBasis(k)
+    X, Y = O.Operator(b, bk, x.to(dt).t()), O.Operator(b, bk, y)
+    graded = np.asfortranarray(a.copy())
+    graded[0] *= (2.0 ** -(30.0 * np.arange(n) / n)).astype(a.real.dtype)
+    ms = []
+    for m in (a, graded):
+        op, best = O.Operator(b, b, m), np.inf
+        for _ in range(6):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            for _ in range(4):
+                mul_(Y, op, X, arith="ff" if form == "ff" else None)
+            e[1].record()
+            torch.cuda.synchronize()
+            best = min(best, e[0].elapsed_time(e[1]) / 4)
+        ms.append(best)
+    # three launches that find nothing to do beside kernels of 50 us and more
+    assert ms[0] < 2 * ms[1], ms
