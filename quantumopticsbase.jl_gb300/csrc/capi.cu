@@ -43,11 +43,27 @@ void* Workspace::get(size_t slot, size_t bytes) {
   if (slots.size() <= slot) slots.resize(slot + 1);
   DeviceBuf& d = slots[slot];
   if (d.bytes < bytes) {
+#ifdef QOB_DEBUG_BOUNDS
+    if (bytes > limit) fail(QOB_ERR_OOM, "workspace limit");
+#endif
     // buffers are reused across calls; wait for work that may still use the old one
     QOB_CUDA(cudaDeviceSynchronize());
     d.alloc(bytes + bytes / 4);
   }
   return d.p;
+}
+
+void* Workspace::try_get(size_t slot, size_t bytes, cudaStream_t s) {
+  if (slots.size() > slot && slots[slot].bytes >= bytes) return slots[slot].p;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  QOB_CUDA(cudaStreamIsCapturing(s, &cs));
+  if (cs != cudaStreamCaptureStatusNone) return nullptr;
+  try {
+    return get(slot, bytes);
+  } catch (const Error& e) {
+    if (e.code != QOB_ERR_OOM) throw;
+    return nullptr;
+  }
 }
 
 Context::~Context() {
@@ -139,13 +155,15 @@ void apply_plan(Context& ctx, Plan& P, c128 alpha, const void* x, int64_t xes, i
       xm.st = xcs;
       ym.st = ycs;
       FmaGate gate;
+      const void* xin = x;
+      void* xs = P.ff ? ctx.ws.get(ws + 1, (size_t)((P.n - 1) * xes + (ncols - 1) * xcs + 1) * 16) : nullptr;
       if (!(form == QOB_C64 ? ctx.fp32_tensor : ctx.fp64_tensor && !P.ff) && slices_pay(form, d.m, d.n, ncols, false) &&
-          slice_ready(d.sl, form, d.a.p, d.m, d.n, slice_swap(yes, ym, ncols), s))
+          slice_ready(d.sl, form, d.a.p, d.m, d.n, slice_swap(yes, ym, ncols), s)) {
+        reserve_dense(P.precision, d.m, d.n, ncols, P.ff, ctx.ws, ws);  // before the planes take what is free
         gate = launch_slices(d.sl, form, ad, x, xes, xm, b, y, yes, ym, ncols, s, &ctx.ws, ws + 2,
                              static_cast<unsigned*>(ctx.status.p), ctx.num_sms, ctx.pdl);
-      const void* xin = x;
+      }
       if (P.ff) {
-        void* xs = ctx.ws.get(ws + 1, (size_t)((P.n - 1) * xes + (ncols - 1) * xcs + 1) * 16);
         launch_ff_split(x, P.n, ncols, xes, xcs, xs, s, gate.any);
         xin = xs;
       }
@@ -203,13 +221,13 @@ void apply_plan(Context& ctx, Plan& P, c128 alpha, const void* x, int64_t xes, i
         auto mode_product = [&](c128 bk, void* out) {
           unsigned* status = static_cast<unsigned*>(ctx.status.p);
           FmaGate gate;
+          const void* sin = src;
+          const int64_t len_in = prod_range(cur, 0, cur.size());
+          void* xs = ffs ? ctx.ws.get(ws + 2, (size_t)((len_in - 1) * ses + (ncols - 1) * scs + 1) * 16) : nullptr;
           if (slices)
             gate = launch_slices(st.sl, form, ak, src, s1 * ses, xm, bk, out, s1 * out_es, ym, pcols, s, &ctx.ws, ws + 3,
                                  status, ctx.num_sms, ctx.pdl);
-          const void* sin = src;
           if (ffs) {
-            const int64_t len_in = prod_range(cur, 0, cur.size());
-            void* xs = ctx.ws.get(ws + 2, (size_t)((len_in - 1) * ses + (ncols - 1) * scs + 1) * 16);
             launch_ff_split(src, len_in, ncols, ses, scs, xs, s, gate.any);
             sin = xs;
           }
@@ -826,6 +844,14 @@ int qob_op_set_tile(qob_ctx* ctx, qob_op* op, int side, int dtype, int vectors_p
 }
 
 #ifdef QOB_DEBUG_BOUNDS
+// Bounds-checked build only: workspace slots that would grow beyond `bytes` fail as they do
+// without memory (0: no limit).
+int qob_debug_limit_workspace(qob_ctx* ctx, size_t bytes) {
+  if (!ctx) return QOB_ERR_ARG;
+  ctx->c.ws.limit = bytes ? bytes : SIZE_MAX;
+  return QOB_OK;
+}
+
 // Bounds-checked build only: moves the input offset of the first stored entry
 // with a nonzero value of op's compiled gather (side, dtype) by col_shift, so
 // that a test can watch the device checks catch an index out of range.

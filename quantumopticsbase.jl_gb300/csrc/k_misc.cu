@@ -419,11 +419,16 @@ int dense_kchunks(int64_t m, int64_t n, int64_t ncols, int tc) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(kch, 65535));
 }
 
+// kets per thread
+int dense_tile(int64_t ncols, bool ff) {
+  return ncols >= 8 && !ff ? 8 : ncols >= 4 ? 4 : ncols >= 2 ? 2 : 1;
+}
+
 template <typename CT, typename R>
 void dense_typed(const void* a, int64_t m, int64_t n, c128 alpha, const void* x, int64_t xes, int64_t xcs,
                  c128 beta, void* y, int64_t yes, int64_t ycs, int64_t ncols, Workspace* ws, int slot,
                  cudaStream_t s, const FmaGate& gate) {
-  const int tc = ncols >= 8 ? 8 : ncols >= 4 ? 4 : ncols >= 2 ? 2 : 1;
+  const int tc = dense_tile(ncols, false);
   int kch = ws ? dense_kchunks(m, n, ncols, tc) : 1;
   CT* part = nullptr;
   if (kch > 1) part = static_cast<CT*>(ws->get(slot, (size_t)kch * ncols * m * sizeof(CT)));
@@ -452,7 +457,7 @@ void dense_typed(const void* a, int64_t m, int64_t n, c128 alpha, const void* x,
 void dense_ff(const void* a, int64_t m, int64_t n, c128 alpha, const void* x, int64_t xes, int64_t xcs,
               c128 beta, void* y, int64_t yes, int64_t ycs, int64_t ncols, Workspace* ws, int slot,
               cudaStream_t s, const FmaGate& gate) {
-  const int tc = ncols >= 4 ? 4 : ncols >= 2 ? 2 : 1;
+  const int tc = dense_tile(ncols, true);
   int kch = ws ? dense_kchunks(m, n, ncols, tc) : 1;
   double2* part = nullptr;
   if (kch > 1) part = static_cast<double2*>(ws->get(slot, (size_t)kch * ncols * m * sizeof(double2)));
@@ -478,6 +483,12 @@ void dense_ff(const void* a, int64_t m, int64_t n, c128 alpha, const void* x, in
   }
 }
 }  // namespace
+
+void reserve_dense(int precision, int64_t m, int64_t n, int64_t ncols, bool ff, Workspace& ws, int slot) {
+  ncols = std::min<int64_t>(ncols, 65535 * 8);  // a launch's
+  const int kch = dense_kchunks(m, n, ncols, dense_tile(ncols, ff));
+  if (kch > 1) ws.get(slot, (size_t)kch * ncols * m * (precision == QOB_C128 ? 16 : 8));
+}
 
 void launch_dense(int precision, const void* a, int64_t m, int64_t n, c128 alpha, const void* x,
                   int64_t xes, int64_t xcs, c128 beta, void* y, int64_t yes, int64_t ycs,

@@ -962,12 +962,16 @@ FmaGate run_slices(const SliceDense& d, bool swap, const void* xv, int64_t xes, 
   const SlicePlanes& pl = swap ? d.nside : d.mside;
   const SliceSide* sides = static_cast<const SliceSide*>(pl.sides.p);
   const size_t bbytes = (size_t)vt * nkb * (swap ? C::kA : C::kB), ebytes = ((size_t)vt * (nch * (tile + 1) + 1) + 1) * sizeof(int);
-  unsigned char* w = static_cast<unsigned char*>(ws->get(slot, bbytes + ebytes));
+  unsigned char* w = static_cast<unsigned char*>(ws->try_get(slot, bbytes + ebytes, s));
+  if (!w) return FmaGate();
   int* exps = reinterpret_cast<int*>(w + bbytes);
   int* flags = exps + vt * nch * tile;
   int *left = flags + vt * nch, *any = left + vt;
   V* part = nullptr;
-  if (per % nch != 0) part = static_cast<V*>(ws->get(slot + 1, (size_t)rtiles * smax * H * HM * sizeof(V)));
+  if (per % nch != 0) {
+    part = static_cast<V*>(ws->try_get(slot + 1, (size_t)rtiles * smax * H * HM * sizeof(V), s));
+    if (!part) return FmaGate();
+  }
   if (swap)
     run_split<FORM, kSlRows, true, V>(x, d.n, xes, xm, ncols, vt, nkb, w, exps, flags, any, sides, nullptr, s, pdl);
   else

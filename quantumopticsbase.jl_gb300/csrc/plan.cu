@@ -841,9 +841,6 @@ static std::unique_ptr<Plan> compile_sum(Context& ctx, const NodeP& root, int si
             for (int64_t row = 0; row < r.rows; ++row)
               for (int64_t p = r.ptr[row]; p < r.ptr[row + 1]; ++p) a[row + r.col[p] * st.dout] = r.val[p];
             upload_matrix(st.a, a, *P);
-            // planes for contiguous kets: their vectors lie side by side unless the site is the first
-            if (!tr && !st.eye && st.dout >= kSliceMin && st.din >= kSliceMin)
-              slice_ready(st.sl, precision, st.a.p, st.dout, st.din, st.site != 0, 0);
             mp.steps.push_back(std::move(st));
           }
           // non-square subsystems without factors: explicit isometries (:491-514)
@@ -890,8 +887,6 @@ static std::unique_ptr<Plan> compile_sum(Context& ctx, const NodeP& root, int si
               a[i + j * dp.m] = v;
             }
           upload_matrix(dp.a, a, *P);
-          if (!tr && dp.m >= kSliceMin && dp.n >= kSliceMin)
-            slice_ready(dp.sl, precision, dp.a.p, dp.m, dp.n, false, 0);
           P->dense.push_back(std::move(dp));
           break;
         }

@@ -318,8 +318,8 @@ struct TcColMap {
   int64_t s1 = 1, s3 = 1, sa = 0, sb = 0, st = 0;
 };
 
-// The digit planes of a dense matrix (k_slice.cu) as either side of the product:
-// the one that contiguous kets take made with the plan, the other on first use.
+// The digit planes of a dense matrix (k_slice.cu) as either side of the product, each made by the
+// first call that takes it: an operator that meets single kets only has none.
 struct SlicePlanes {
   int state = 0;  // 0: not made, 1: ready, -1: the matrix is left to the FMA kernels
   DeviceBuf planes, exps;
@@ -411,6 +411,12 @@ struct Plan {
 struct Workspace {
   std::vector<DeviceBuf> slots;
   void* get(size_t slot, size_t bytes);
+  // the same for work that has another way: null where there is no memory for it, or the
+  // slot would grow while s is captured
+  void* try_get(size_t slot, size_t bytes, cudaStream_t s);
+#ifdef QOB_DEBUG_BOUNDS
+  size_t limit = SIZE_MAX;  // bytes of a slot (qob_debug_limit_workspace)
+#endif
 };
 
 struct Context {
@@ -495,6 +501,8 @@ void launch_dense(int precision, const void* a, int64_t m, int64_t n, c128 alpha
                   int64_t xes, int64_t xcs, c128 beta, void* y, int64_t yes, int64_t ycs,
                   int64_t ncols, cudaStream_t s, Workspace* ws = nullptr, int slot = 0, bool ff = false,
                   bool dmma = false, FmaGate gate = {});
+// Slot `slot` as launch_dense will need it.
+void reserve_dense(int precision, int64_t m, int64_t n, int64_t ncols, bool ff, Workspace& ws, int slot);
 // The same on the FP64 tensor cores (k_dmma.cu; ComplexF64 only).
 void launch_dense_dmma(const void* a, int64_t m, int64_t n, c128 alpha, const void* x, int64_t xes, int64_t xcs,
                        c128 beta, void* y, int64_t yes, int64_t ycs, int64_t ncols, cudaStream_t s, Workspace* ws,
@@ -522,6 +530,7 @@ bool launch_gemm_tc(const TcDense& d, c128 alpha, const void* x, int64_t xes, co
 // makes the matrix's planes for it if they are not there yet (not inside a capture)
 // and says whether they can be used.  Workspace slots slot, slot + 1.  The columns of
 // the tiles that the returned gate names are not written: the FMA kernels follow with it.
+// Without room for the vectors' planes nothing is done and the gate is open to every column.
 constexpr int64_t kSliceMin = 32;  // rows and columns from which a matrix gets planes
 bool slice_swap(int64_t yes, const TcColMap& ym, int64_t ncols);
 bool slice_ready(SliceDense& d, int form, const void* a, int64_t m, int64_t n, bool swap, cudaStream_t s);
