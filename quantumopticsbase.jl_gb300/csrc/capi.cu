@@ -853,7 +853,8 @@ int qob_debug_limit_workspace(qob_ctx* ctx, size_t bytes) {
 }
 
 // Bounds-checked build only: moves the input offset of the first stored entry
-// with a nonzero value of op's compiled gather (side, dtype) by col_shift, so
+// with a nonzero value of op's compiled gather (side, dtype) by col_shift, and with it the
+// flip of its group in a plan of the flip form (col_shift a power of two there), so
 // that a test can watch the device checks catch an index out of range.
 int qob_debug_shift_slot(qob_ctx* ctx, qob_op* op, int side, int dtype, int col_shift) {
   return guard(ctx, [&] {
@@ -878,6 +879,13 @@ int qob_debug_shift_slot(qob_ctx* ctx, qob_op* op, int side, int dtype, int col_
       col += col_shift;
       std::memcpy(e, &col, 4);
       QOB_CUDA(cudaMemcpy(g.ell.p, h.data(), h.size(), cudaMemcpyHostToDevice));
+      if (g.multi) {
+        std::vector<int4> rec(2 * (size_t)g.ngroups);
+        QOB_CUDA(cudaMemcpy(rec.data(), g.mrec.p, rec.size() * sizeof(int4), cudaMemcpyDeviceToHost));
+        for (size_t r = 0; r < rec.size(); r += 2)
+          if ((int)i >= rec[r].z && (int)i < rec[r].z + rec[r].w) rec[r + 1].x ^= col_shift;
+        QOB_CUDA(cudaMemcpy(g.mrec.p, rec.data(), rec.size() * sizeof(int4), cudaMemcpyHostToDevice));
+      }
       return;
     }
     fail(QOB_ERR_UNSUPPORTED, "no stored entry with a nonzero value");

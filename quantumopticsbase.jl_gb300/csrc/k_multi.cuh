@@ -340,10 +340,12 @@ __device__ __forceinline__ void combine_block(typename Cx<R>::T* yp, int64_t yes
 // record is f, has a stored entry.
 template <typename R, int NI, bool IM, int LOW>
 __device__ __forceinline__ void low_group(typename Multi<R>::Acc (&acc)[NI], const typename Multi<R>::X (&u)[NI],
-                                          const int4& f, const typename Ell<R, true>::T* ell, uint32_t J0) {
+                                          const int4& f, const typename Ell<R, true>::T* ell, uint32_t J0,
+                                          const GatherView& g) {
   using M = Multi<R>;
 #pragma unroll
   for (int e = 0; e < NI; ++e) {
+    if (kDebugBounds && out_of_range((int64_t)f.z + multi_row<true>(f, J0 + e), g.ell_slots, g.status)) continue;
     const auto v = Ell<R, true>::v(ell[f.z + multi_row<true>(f, J0 + e)]);
     int turn = nz(v) ? 1 : 0;
     if constexpr (std::is_same<R, double>::value) {
@@ -395,10 +397,13 @@ __global__ void __launch_bounds__(kFlipThreads, MultiOcc<R>::value) k_gather_m(G
     int4 f = g.mrec[2 * i];
     const int rows = f.w;  // at most 32
     f.w = 0;
-    for (int r = 0; r < rows; ++r) f.w |= (nz(Ell<R, true>::v(ell[f.z + r])) ? 1 : 0) << r;
+    for (int r = 0; r < rows; ++r) {
+      if (kDebugBounds && out_of_range((int64_t)f.z + r, g.ell_slots, g.status)) continue;
+      f.w |= (nz(Ell<R, true>::v(ell[f.z + r])) ? 1 : 0) << r;
+    }
     rec[i] = f;
     const int4 q = g.mrec[2 * i + 1];
-    fl[i] = M::record((uint32_t)q.x, Ell<R, true>::v(ell[q.y]));
+    fl[i] = M::record((uint32_t)q.x, Ell<R, true>::v(ell[kDebugBounds && out_of_range(q.y, g.ell_slots, g.status) ? 0 : q.y]));
   }
   if (g.ell_smem) {
     uint32_t* dst = reinterpret_cast<uint32_t*>(smem_raw + (size_t)g.ngroups * (sizeof(int4) + 16));
@@ -433,6 +438,18 @@ __global__ void __launch_bounds__(kFlipThreads, MultiOcc<R>::value) k_gather_m(G
     activity(std::true_type{});
   else
     activity(std::false_type{});
+  if (kDebugBounds) {  // groups whose block of inputs starts or ends outside the vector, or is not aligned, do not run
+    auto inside = [&](uint32_t act, const Rec* r0) {
+      for (uint32_t a = act; a; a &= a - 1) {
+        const int b = __ffs((int)a) - 1;
+        const uint32_t p = J0 ^ r0[b].flip;
+        if (out_of_range((p & (NI - 1)) ? -1 : (int64_t)p + NI - 1, g.n, g.status)) act &= ~(1u << b);
+      }
+      return act;
+    };
+    act_re = inside(act_re, fl + nlow);
+    if constexpr (PH) act_im = inside(act_im, fl + nre);
+  }
   DT d[NI];
   if (g.has_diag) {
 #pragma unroll
@@ -467,13 +484,14 @@ __global__ void __launch_bounds__(kFlipThreads, MultiOcc<R>::value) k_gather_m(G
       for (int k = k0; k < k1; ++k) {
         const int4 f = rec[k];
         const uint32_t flip = fl[k].flip;
+        if (kDebugBounds && out_of_range((int64_t)(J0 ^ (flip & ~(uint32_t)(NI - 1))) + NI - 1, g.n, g.status)) continue;
         X u[NI];
         ld_block<X, NI, WIDE>(xb + (int64_t)(J0 ^ (flip & ~(uint32_t)(NI - 1))) * xes, xes, u);
         switch (flip & (NI - 1)) {
-          case 0: low_group<R, NI, IM, 0>(acc, u, f, ell, J0); break;
-          case 1: low_group<R, NI, IM, 1>(acc, u, f, ell, J0); break;
-          case 2: if constexpr (NI > 2) low_group<R, NI, IM, 2>(acc, u, f, ell, J0); break;
-          default: if constexpr (NI > 2) low_group<R, NI, IM, 3>(acc, u, f, ell, J0);
+          case 0: low_group<R, NI, IM, 0>(acc, u, f, ell, J0, g); break;
+          case 1: low_group<R, NI, IM, 1>(acc, u, f, ell, J0, g); break;
+          case 2: if constexpr (NI > 2) low_group<R, NI, IM, 2>(acc, u, f, ell, J0, g); break;
+          default: if constexpr (NI > 2) low_group<R, NI, IM, 3>(acc, u, f, ell, J0, g);
         }
       }
     };

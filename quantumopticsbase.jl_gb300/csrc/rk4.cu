@@ -145,8 +145,14 @@ __global__ void __launch_bounds__(kRk4Threads, 7) k_rk4_list(Rk4Args a, int cap)
       uint32_t r, sub;
       gather::local_row(G, (uint32_t)j, r, sub);
       for (int k = 0; k < G.width; ++k) {
+        if (gather::kDebugBounds &&
+            gather::out_of_range((int64_t)G.ell_off + (int64_t)r * G.width + k, g.ell_slots, g.status))
+          continue;
         const ET e = ell[G.ell_off + (int64_t)r * G.width + k];
         const VT v = gather::Ell<R, REALV>::v(e);
+        if (gather::kDebugBounds && gather::nz(v) &&
+            gather::out_of_range((int64_t)((uint32_t)j - sub) + e.col, g.n, g.status))
+          continue;
         if (gather::nz(v) && ne < cap) {
           vals[ne * kRk4Threads] = v;
           idx[ne * kRk4Threads] = (int)((uint32_t)j - sub) + e.col;
