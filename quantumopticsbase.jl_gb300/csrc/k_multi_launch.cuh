@@ -64,7 +64,7 @@ void launch_multi(const GatherView& v, const void* x, int64_t xes, int64_t xcs, 
   if (!std::is_same<R, double>::value) {
     constexpr int NI = flip_block(std::is_same<R, float>::value ? QOB_C64 : QOB_C128, std::is_same<R, DF>::value);
     const int64_t blocks = (v.m * ls / (NI * kFlipThreads) + 1) * ((ncols + ls - 1) / ls);
-    kper = (int)std::max<int64_t>(1, std::min<int64_t>(std::is_same<R, float>::value ? 3 : 4, blocks / 1064 + 1));
+    kper = (int)std::max<int64_t>(1, std::min<int64_t>(std::is_same<R, float>::value ? 3 : 4, blocks / (7 * current_sms()) + 1));
   }
 #define QOB_M_CALL(W, B) launch_m<R, VM, W, B>(v, ls, kper, x, xes, xcs, y, yes, ycs, ncols, a, b, s)
   if (is_zero(beta))
