@@ -240,7 +240,8 @@ int qob_op_tune(qob_ctx* ctx, qob_op* op, int side, int dtype, int64_t ncols, do
  * the flip form runs without a tuned shape (every merged group flips a fixed set
  * of index bits of at most two runs of power-of-two subsystems, with one value:
  * Pauli strings, bonds and ladder products of spin chains, either side and any
- * strides; it sizes itself); *chosen has bit 29 set when it won.  The staged tiles: blocks of 256 threads that copy tiles of 2^bits
+ * strides; it sizes itself), -1 where a call of this size does not run it;
+ * *chosen has bit 29 set when it won.  The staged tiles: blocks of 256 threads that copy tiles of 2^bits
  * consecutive indices of their kets into shared memory, for (bits, vectors per
  * thread, vector sets per warp) = (10,1,1) (10,2,1) (9,4,1) (11,1,1) (11,2,1)
  * (12,1,1) (9,1,4) (8,1,16) (8,2,8) (9,2,4) (10,1,4) (7,2,16); -1 when not

@@ -696,7 +696,7 @@ int tune_impl(qob_ctx* ctx, qob_op* op, int side, int dtype, int64_t ncols, doub
           tb = tbits_c[i];
           if (!tiles_ok || tb > mbits || tc * ls > ncols) continue;
         } else if (k == kCands - 1) {
-          if (!g.multi) continue;
+          if (!g.multi || !flip_runs(g.m, ncols, xes, yes)) continue;
           tc = blk = 0;  // no shape of the other kernels: the flip form's own
           ls = 1;
         } else {

@@ -1150,8 +1150,6 @@ void launch_tile_tc(const GatherView& v, int tc, const void* x, int64_t xcs, voi
   }
 }
 
-constexpr int64_t kFlipMin = 16384;  // elements of a call from which k_gather_m runs
-
 // k_gather_m on this call (k_multi_{f64,f32,df}.cu)
 template <typename R, int VM>
 void launch_multi(const GatherView& v, const void* x, int64_t xes, int64_t xcs, void* y, int64_t yes, int64_t ycs,
@@ -1239,11 +1237,8 @@ void dispatch_beta(const GatherView& v, const SiteTable& st, int tc, const void*
 template <typename R>
 void dispatch(const GatherView& v, const SiteTable& st, int tc, const void* x, int64_t xes, int64_t xcs,
               void* y, int64_t yes, int64_t ycs, int64_t ncols, c128 alpha, c128 beta, cudaStream_t s) {
-  // the flip form's kernel, unless a shape of the others was tuned or set.  A
-  // ket of a few thousand entries is faster with one index per thread (10 spins,
-  // ComplexF64, 4.7 against 5.2 us; 12 spins, double-float, 6.7 against 7.5);
-  // strided vectors gain at every size.
-  if (v.multi && v.automatic && ncols <= INT32_MAX && (v.m * ncols >= kFlipMin || xes != 1 || yes != 1)) {
+  // the flip form's kernel, unless a shape of the others was tuned or set
+  if (v.multi && v.automatic && flip_runs(v.m, ncols, xes, yes)) {
     if (v.real_vals)
       launch_multi<R, kReal>(v, x, xes, xcs, y, yes, ycs, ncols, alpha, beta, s);
     else
