@@ -67,6 +67,7 @@
 #include "k_gather.cuh"  // double-float helpers
 #include "launch.cuh"
 #include "qob_internal.h"
+#include "tcgen05.cuh"
 
 namespace qob {
 
@@ -74,42 +75,11 @@ namespace {
 
 constexpr int kSlChunk = 16;      // k steps of 16 in a chunk, at most
 constexpr int kSlRows = 128;      // real matrix rows of a tile
-constexpr int kSlPolls = 1 << 21;
-constexpr unsigned kSlErrTimeout = 1u;
 
 // The chunks of nkb k steps are of equal length but for one step: chunk c is the k
 // steps from chunk_start(c) to chunk_start(c + 1).
 __host__ __device__ inline int chunk_start(int c, int nkb, int nch) { return (int)((int64_t)c * nkb / nch); }
 
-__device__ __forceinline__ uint32_t saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void bar_init(uint64_t* b, unsigned n) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(b)), "r"(n) : "memory");
-}
-__device__ __forceinline__ void bar_expect(uint64_t* b, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(saddr(b)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bar_arrive(uint64_t* b) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(b)) : "memory");
-}
-__device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t parity) {
-  for (int i = 0; i < kSlPolls; ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(saddr(b)), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if (i > 64) __nanosleep(32);
-  }
-  return false;
-}
-__device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* b) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   saddr(dst)),
-               "l"(src), "r"(bytes), "r"(saddr(b))
-               : "memory");
-}
 // K-major operand without swizzle: core matrices of 8 rows x 16 bytes, the two of
 // a k step 128 bytes apart, 8-row groups 256 bytes apart; descriptor version 1
 __device__ __forceinline__ uint64_t plane_desc(const void* p) {
@@ -122,10 +92,6 @@ __device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t ad, uint64_t bd, u
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
       "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
       : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint64_t* b) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(saddr(b))
-               : "memory");
 }
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[4]) {  // completion: tcgen05.wait::ld
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
@@ -256,13 +222,6 @@ __host__ __device__ inline float digit_error(const SliceSide& a, const SliceSide
   return t > 1024.f ? 3e38f : a.n1 + x.n1 + 1.01f * t;
 }
 
-__device__ __forceinline__ int64_t col_offset(const TcColMap& m, int64_t c) {
-  if (m.s1 == 1 && m.s3 == 1) return c * m.st;
-  const uint32_t cc = (uint32_t)c, s1 = (uint32_t)m.s1, s3 = (uint32_t)m.s3;
-  const uint32_t a = cc % s1, q = cc / s1;
-  return (int64_t)a * m.sa + (int64_t)(q % s3) * m.sb + (int64_t)(q / s3) * m.st;
-}
-
 // Digit planes of one tile's chunk: ROWS / 2 vectors (columns of x, or rows of the
 // matrix with INTER) x up to 256 contracted indices.  blockIdx.x: tile, blockIdx.y:
 // chunk.  exps[(tile nch + chunk) ROWS / 2 + vector]: the power of two above its
@@ -297,7 +256,7 @@ __global__ void __launch_bounds__(split_threads(ROWS)) k_slice_split(const IN* _
   if (any && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) *any = 0;  // set by the GEMM
   if (threadIdx.x < kLevels) side.c[threadIdx.x] = kSlChunk * 16;
   if (threadIdx.x < ROWS) cnt_hi[threadIdx.x] = cnt_lo[threadIdx.x] = sum1[threadIdx.x] = sum2[threadIdx.x] = 0u;
-  if (threadIdx.x < H) off[threadIdx.x] = v0 + threadIdx.x < nvec ? col_offset(map, v0 + threadIdx.x) : -1;
+  if (threadIdx.x < H) off[threadIdx.x] = v0 + threadIdx.x < nvec ? tc_col_offset(map, v0 + threadIdx.x) : -1;
   auto stage = [&](int b0) {  // k steps b0 .. of the chunk
     const int nk = min(sub, nks - b0) * 16;
     __syncthreads();
@@ -818,8 +777,8 @@ __global__ void __launch_bounds__(SlCfg<FORM, BN>::kThreads, 1)
         const int64_t seg = (int64_t)blockIdx.x - (rt * nch) / per;  // segment in the row tile
         // y offsets: of this lane's M-side row, and in lane c of the warp's N-side row c
         const int64_t cl = ct * H + half * KQ + lane;
-        const int64_t moff = i >= m ? 0 : swap ? col_offset(ym, i) : i * yes;
-        const int64_t noff = lane >= KQ || cl >= ncols ? 0 : swap ? cl * yes : col_offset(ym, cl);
+        const int64_t moff = i >= m ? 0 : swap ? tc_col_offset(ym, i) : i * yes;
+        const int64_t noff = lane >= KQ || cl >= ncols ? 0 : swap ? cl * yes : tc_col_offset(ym, cl);
         const bool reads = whole && (beta_re || beta_im);
         T own[KQ];  // y's component of this lane, all loaded before the first is used
 #pragma unroll
@@ -863,7 +822,7 @@ __global__ void __launch_bounds__(SlCfg<FORM, BN>::kThreads, 1)
     }
     if (!ok) {
       atomicExch(abort_flag, 1);
-      if (lane == 0 && status) atomicOr(status, kSlErrTimeout);
+      if (lane == 0 && status) atomicOr(status, kTcErrTimeout);
     }
   }
   if (warp == 1 && lane == 0) bar_wait(fin, 0);
@@ -911,7 +870,7 @@ __global__ void k_slice_reduce(const typename Sl<FORM>::V* __restrict__ part, co
       re += p.x;
       im += p.y;
     }
-    axpby_out(y + (swap ? cg * yes + col_offset(ym, i) : i * yes + col_offset(ym, cg)), re, im, alpha, beta);
+    axpby_out(y + (swap ? cg * yes + tc_col_offset(ym, i) : i * yes + tc_col_offset(ym, cg)), re, im, alpha, beta);
   }
 }
 
