@@ -919,7 +919,7 @@ FmaGate run_slices(const SliceDense& d, bool swap, const void* xv, int64_t xes, 
   const int smax = (int)((nch - 1) / per + 2);
   const int64_t tile = swap ? HM : H;  // vectors of a tile
   const SlicePlanes& pl = swap ? d.nside : d.mside;
-  const SliceSide* sides = static_cast<const SliceSide*>(pl.sides.p);
+  const SliceSide* sides = static_cast<const SliceSide*>(pl.sides);
   const size_t bbytes = (size_t)vt * nkb * (swap ? C::kA : C::kB), ebytes = ((size_t)vt * (nch * (tile + 1) + 1) + 1) * sizeof(int);
   unsigned char* w = static_cast<unsigned char*>(ws->try_get(slot, bbytes + ebytes, s));
   if (!w) return FmaGate();
@@ -935,10 +935,10 @@ FmaGate run_slices(const SliceDense& d, bool swap, const void* xv, int64_t xes, 
     run_split<FORM, kSlRows, true, V>(x, d.n, xes, xm, ncols, vt, nkb, w, exps, flags, any, sides, nullptr, s, pdl);
   else
     run_split<FORM, BN, false, V>(x, d.n, xes, xm, ncols, vt, nkb, w, exps, flags, any, sides, nullptr, s, pdl);
-  const unsigned char* mp = swap ? w : static_cast<const unsigned char*>(pl.planes.p);
-  const unsigned char* np = swap ? static_cast<const unsigned char*>(pl.planes.p) : w;
-  const int* me = swap ? exps : static_cast<const int*>(pl.exps.p);
-  const int* ne = swap ? static_cast<const int*>(pl.exps.p) : exps;
+  const unsigned char* mp = swap ? w : pl.planes;
+  const unsigned char* np = swap ? pl.planes : w;
+  const int* me = swap ? exps : pl.exps;
+  const int* ne = swap ? pl.exps : exps;
   auto kern = k_slice_gemm<FORM, BN>;
   QOB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem));
   // the launches behind the split kernel overlap with the one before (pdl_enter, pdl_wait): the
@@ -970,32 +970,31 @@ void build_slices(SliceDense& d, bool swap, const void* a, cudaStream_t s) {
   SlicePlanes& pl = swap ? d.nside : d.mside;
   const int nch = (d.nkb + kSlChunk - 1) / kSlChunk;
   const int64_t half = swap ? kSwapBN / 2 : kSlRows / 2, tiles = (d.m + half - 1) / half;
-  pl.planes.alloc((size_t)tiles * d.nkb * S * (swap ? kSwapBN * 32 : kSlRows * 16));
-  pl.exps.alloc((size_t)tiles * nch * (half + 1) * sizeof(int));
-  int* exps = static_cast<int*>(pl.exps.p);
-  int* flags = exps + tiles * nch * half;
-  DeviceBuf own;
-  own.alloc((size_t)(tiles * nch) * sizeof(SliceSide));
-  auto* tile_sides = static_cast<SliceSide*>(own.p);
+  // one allocation: planes, exponents, the chunks' sides, then what the host looks at, flags and
+  // sides of each tile's chunks
+  const size_t nt = (size_t)(tiles * nch), pbytes = (size_t)tiles * d.nkb * S * (swap ? kSwapBN * 32 : kSlRows * 16);
+  pl.buf.alloc(pbytes + nt * half * sizeof(int) + (nt + nch) * sizeof(SliceSide) + nt * sizeof(int));
+  unsigned char* planes = static_cast<unsigned char*>(pl.buf.p);
+  int* exps = reinterpret_cast<int*>(planes + pbytes);
+  auto* sides = reinterpret_cast<SliceSide*>(exps + nt * half);
+  auto* tile_sides = sides + nch;
+  int* flags = reinterpret_cast<int*>(tile_sides + nt);
   TcColMap map;  // "vectors" = matrix rows, one element apart; contracted index = column, m apart
   map.st = 1;
   const auto* m = static_cast<const typename Sl<FORM>::M*>(a);
   if (swap)
     run_split<FORM, kSwapBN, false, typename Sl<FORM>::M>(m, d.n, d.m, map, d.m, tiles, d.nkb,
-                                                          static_cast<unsigned char*>(pl.planes.p), exps, flags,
-                                                          nullptr, nullptr, tile_sides, s, false);
+                                                          planes, exps, flags, nullptr, nullptr, tile_sides, s, false);
   else
     run_split<FORM, kSlRows, true, typename Sl<FORM>::M>(m, d.n, d.m, map, d.m, tiles, d.nkb,
-                                                         static_cast<unsigned char*>(pl.planes.p), exps, flags,
-                                                         nullptr, nullptr, tile_sides, s, false);
-  std::vector<int> f((size_t)(tiles * nch));
-  std::vector<SliceSide> q((size_t)(tiles * nch)), worst((size_t)nch);
-  QOB_CUDA(cudaMemcpyAsync(f.data(), flags, f.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
-  QOB_CUDA(cudaMemcpyAsync(q.data(), tile_sides, q.size() * sizeof(SliceSide), cudaMemcpyDeviceToHost, s));
+                                                         planes, exps, flags, nullptr, nullptr, tile_sides, s, false);
+  std::vector<SliceSide> q(nt + (nt * sizeof(int) + sizeof(SliceSide) - 1) / sizeof(SliceSide)), worst((size_t)nch);
+  QOB_CUDA(cudaMemcpyAsync(q.data(), tile_sides, nt * (sizeof(SliceSide) + sizeof(int)), cudaMemcpyDeviceToHost, s));
   QOB_CUDA(cudaStreamSynchronize(s));
-  pl.state = 1;
-  for (int v : f)
-    if (v) pl.state = -1;
+  const int* f = reinterpret_cast<const int*>(q.data() + nt);
+  int state = 1;
+  for (size_t i = 0; i < nt; ++i)
+    if (f[i]) state = -1;
   for (int ch = 0; ch < nch; ++ch) {
     SliceSide& w = worst[(size_t)ch] = q[(size_t)ch];
     for (int64_t t = 1; t < tiles; ++t) {
@@ -1010,14 +1009,18 @@ void build_slices(SliceDense& d, bool swap, const void* a, cudaStream_t s) {
     const SliceSide ones{0.5f * (float)n, 0.f, {n, n, n, n, n, n}};
     float least = 0.f;
     for (int k = 0; k < kLevels * kLevels; ++k) least += overlap(w, ones, n, k / kLevels, k % kLevels);
-    if (digit_error(w, ones) > kSlLimit<FORM> * least) pl.state = -1;
+    if (digit_error(w, ones) > kSlLimit<FORM> * least) state = -1;
   }
-  if (pl.state > 0) {
-    pl.sides.upload(worst.data(), worst.size() * sizeof(SliceSide));
+  if (state > 0) {
+    QOB_CUDA(cudaMemcpyAsync(sides, worst.data(), worst.size() * sizeof(SliceSide), cudaMemcpyHostToDevice, s));
+    QOB_CUDA(cudaStreamSynchronize(s));  // for calls on any stream
+    pl.planes = planes;
+    pl.exps = exps;
+    pl.sides = sides;
   } else {
-    pl.planes = DeviceBuf();
-    pl.exps = DeviceBuf();
+    pl.buf = DeviceBuf();
   }
+  pl.state = state;
 }
 
 }  // namespace
@@ -1047,8 +1050,7 @@ bool slice_ready(SliceDense& d, int form, const void* a, int64_t m, int64_t n, b
       build_slices<QOB_C64>(d, swap, a, s);
   } catch (const Error& e) {
     if (e.code != QOB_ERR_OOM) throw;
-    pl.planes = DeviceBuf();  // no room for the planes: the FMA kernels
-    pl.exps = DeviceBuf();
+    pl.buf = DeviceBuf();  // no room for the planes: the FMA kernels
     pl.state = -1;
   }
   return pl.state > 0;

@@ -329,8 +329,10 @@ struct TcColMap {
 // first call that takes it: an operator that meets single kets only has none.
 struct SlicePlanes {
   int state = 0;  // 0: not made, 1: ready, -1: the matrix is left to the FMA kernels
-  DeviceBuf planes, exps;
-  DeviceBuf sides;  // per chunk, the worst of the rows (k_slice.cu, SliceSide)
+  DeviceBuf buf;
+  const unsigned char* planes = nullptr;  // in buf
+  const int* exps = nullptr;
+  const void* sides = nullptr;  // per chunk, the worst of the rows (k_slice.cu, SliceSide)
 };
 struct SliceDense {
   int64_t m = 0, n = 0;
