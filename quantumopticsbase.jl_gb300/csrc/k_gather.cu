@@ -73,29 +73,32 @@ __global__ void __launch_bounds__(256) k_ff_split(const double2* __restrict__ x,
     if (*any == 0) return;
   }
   const int64_t total = n * ncols;
-  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x * kSplitPer + threadIdx.x;
-  int64_t o[kSplitPer];
-  double2 v[kSplitPer];
+  int64_t i0 = blockIdx.x * (int64_t)blockDim.x * kSplitPer + threadIdx.x;
+  do {
+    int64_t o[kSplitPer];
+    double2 v[kSplitPer];
 #pragma unroll
-  for (int k = 0; k < kSplitPer; ++k) {
-    const int64_t i = i0 + (int64_t)k * blockDim.x;
-    o[k] = -1;
-    if (i < total) {
-      if (es == 1 && cs == n) {  // contiguous columns (kets): offset = index, no division
-        o[k] = i;
-      } else {
-        int64_t c, e;
-        udivmod(i, n, c, e);
-        o[k] = e * es + c * cs;
+    for (int k = 0; k < kSplitPer; ++k) {
+      const int64_t i = i0 + (int64_t)k * blockDim.x;
+      o[k] = -1;
+      if (i < total) {
+        if (es == 1 && cs == n) {  // contiguous columns (kets): offset = index, no division
+          o[k] = i;
+        } else {
+          int64_t c, e;
+          udivmod(i, n, c, e);
+          o[k] = e * es + c * cs;
+        }
+        v[k] = __ldg(x + o[k]);
       }
-      v[k] = __ldg(x + o[k]);
     }
-  }
 #pragma unroll
-  for (int k = 0; k < kSplitPer; ++k)
-    if (o[k] >= 0) {
-      out[o[k]] = gather::ff_split4(v[k]);
-    }
+    for (int k = 0; k < kSplitPer; ++k)
+      if (o[k] >= 0) {
+        out[o[k]] = gather::ff_split4(v[k]);
+      }
+    i0 += (int64_t)gridDim.x * blockDim.x * kSplitPer;
+  } while (GATED && i0 < total);  // behind a gate the grid is one wave: most often there is nothing to do
 }
 
 // Stored values re-evaluated from the root LazySum's factors: one thread per
@@ -235,7 +238,8 @@ void launch_ff_split(const void* x, int64_t n, int64_t ncols, int64_t es, int64_
                      const int* any) {
   const int64_t total = n * ncols;
   if (total == 0) return;
-  const unsigned blocks = (unsigned)((total + 256 * kSplitPer - 1) / (256 * kSplitPer));
+  unsigned blocks = (unsigned)((total + 256 * kSplitPer - 1) / (256 * kSplitPer));
+  if (any) blocks = std::min(blocks, 8u * (unsigned)gather::current_sms());
   launch_kernel(any != nullptr, any ? k_ff_split<true> : k_ff_split<false>, dim3(blocks), 256u, 0, s,
                 static_cast<const double2*>(x), n, ncols, es, cs, static_cast<float4*>(out), any);
   QOB_LAUNCHED();

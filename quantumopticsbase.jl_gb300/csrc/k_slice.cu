@@ -12,24 +12,29 @@
 // relative to 2^ex(c), both per chunk of at most 256 contracted indices, 8 S - 2 bits
 // below it and truncated there.  The pairs (i, j) of digits with i + j = d < S are summed in
 // one FP32 accumulator, a diagonal, as integers; the S diagonals are added as 64-bit
-// integers and rounded once.  S = 8 in ComplexF64 (62 bits) and double-float, 5 in
-// ComplexF32 (38 bits).
+// integers and rounded once.  S = 8 in ComplexF64 (62 bits), 7 in double-float (54), 4 in
+// ComplexF32 (30).
 //
 // What the digits leave out is small against a row's and a vector's largest
 // components, and the products of those may be absent from a sum: a product is made of
-// digits only where a bound says that nothing is lost.  Per row or vector and chunk the split
+// digits only where a bound says that little is lost.  Per row or vector and chunk the split
 // kernel keeps the sum of the magnitudes, of the digits squared, and how many
 // components reach 2^-1 .. 2^-6 of the power of two.  The first two bound the error
 // (digit_error: the truncation of either side, the diagonals from S on; nothing rounds in an
-// accumulator below 2^24), the counts bound sum |a| |x| from below (overlap).  The error has to be
-// at most 2^-24 of that in ComplexF32, 2^-48 in double-float and 2^-50 in ComplexF64,
-// for every row, vector and chunk, Re and Im apart: no more than the bound of a chain of
-// multiply-adds over 4 terms, and the counts ask for more.  A tile of vectors that fails (graded
-// ones, sparse ones, components that are not finite or far from 1) is left
-// to the FMA kernels: the split kernel flags it, the GEMM does not store it and the
-// FMA kernels, launched behind it, compute the flagged tiles alone (FmaGate).  A matrix that fails with vectors of ones has no
-// planes.  Gaussian entries (matrices of 32 to 4096 rows) reach 0.2 of the limit in ComplexF32
-// and double-float and 0.7 in ComplexF64, and 650 of the 1024 that keep a diagonal exact.
+// accumulator below 2^24), the counts bound sum |a| |x| from below (overlap).  The error's bound has to be
+// at most 8 units (2^-53) of that in ComplexF64, 32 (2^-24) in ComplexF32, 64 (2^-48) in
+// double-float, for every row, vector and chunk, Re and Im apart: what a chain of
+// multiply-adds over 4, 16 and 32 terms is bounded by, where the shortest sums here have 32
+// pairs.  The error itself is far below: over Gaussian, uniform, constant, lognormal, graded,
+// cancelling and sparse entries that pass, 64 or 256 of them (digits and chains emulated on the
+// CPU), 0.3 to 0.9 units in relative l2 in ComplexF32 where the chain has 1.8 to 7, and up to
+// 1 against 16 units of sum |a| |x|.  Gaussian entries (matrices of 32 to 4096 rows) reach 0.9
+// of the limits and 650 of the 1024 that keep a diagonal exact.
+//
+// A tile of vectors that fails (graded ones, sparse ones, components that are not finite or
+// far from 1) is left to the FMA kernels: the split kernel flags it, the GEMM does not store
+// it and the FMA kernels, launched behind it, compute the flagged tiles alone (FmaGate).  A
+// matrix that fails with vectors of ones has no planes.
 //
 // Layout.  The complex product is one real GEMM as in k_tc32.cu: rows 2i, 2i + 1 of
 // a 128-row tile hold Re and Im of matrix row i, rows j and BN/2 + j of a BN-row
@@ -123,13 +128,13 @@ struct Sl<QOB_C128> {
 };
 template <>
 struct Sl<QOB_C128X> {
-  static constexpr int S = 8;
+  static constexpr int S = 7;
   using V = double2;
   using M = float4;
 };
 template <>
 struct Sl<QOB_C64> {
-  static constexpr int S = 5;
+  static constexpr int S = 4;
   using V = float2;
   using M = float2;
 };
@@ -161,18 +166,30 @@ __device__ __forceinline__ long long fixed_point(double v, int e) {
   return __double2hiint(v) < 0 ? -f : f;
 }
 template <int S>
-__device__ __forceinline__ long long fixed_point(float v, int e) {
+__device__ __forceinline__ int fixed_point(float v, int e) {
   const uint32_t hi = mag_hi(v);
   const int ev = (int)(hi >> 23);
   const uint32_t m = (hi & 0x7fffffu) | (ev ? 0x800000u : 0u);
   const int sh = kBits<S> - 24 - (e - ((ev ? ev : 1) - 126));
-  const long long f = sh >= 0 ? (long long)m << sh : sh > -32 ? (long long)(m >> -sh) : 0;
+  const int f = sh >= 0 ? (int)(m << sh) : sh > -32 ? (int)(m >> -sh) : 0;
   return __float_as_int(v) < 0 ? -f : f;
 }
 // All signed digits of f at once: f + sum 128 256^s has the bytes d_s + 128.
 __device__ __forceinline__ uint2 digit_bytes(long long f) {
   const unsigned long long g = (unsigned long long)f + 0x8080808080808080ull;
   return make_uint2((uint32_t)g, (uint32_t)(g >> 32));
+}
+__device__ __forceinline__ uint2 digit_bytes(int f) { return make_uint2((uint32_t)f + 0x80808080u, 0x80808080u); }
+__device__ __forceinline__ unsigned long long magnitude(long long f) { return f < 0 ? -f : f; }
+__device__ __forceinline__ uint32_t magnitude(int f) { return f < 0 ? -f : f; }
+// binary digits above the first of a magnitude's kBits
+template <int S>
+__device__ __forceinline__ int lead(unsigned long long mag) {
+  return __clzll((long long)mag) - (64 - kBits<S>);
+}
+template <int S>
+__device__ __forceinline__ int lead(uint32_t mag) {
+  return __clz((int)mag) - (32 - kBits<S>);
 }
 // digits b of p and q, as two bytes (of d + 128)
 __device__ __forceinline__ uint32_t digit_pair(uint2 p, uint2 q, int b) {
@@ -199,10 +216,10 @@ struct SliceSide {
 };
 constexpr int kLevels = 6;
 
-// Error of the digit products allowed, in 2^-kBits of sum |a| |x|: a unit of the form
-// (2^-24, 2^-48), eight units of 2^-53 in ComplexF64.
+// Bound on the error of the digit products allowed, in 2^-kBits of sum |a| |x|: 8 units of 2^-53 in
+// ComplexF64, 32 of 2^-24 in ComplexF32, 64 of 2^-48 in double-float.
 template <int FORM>
-constexpr float kSlLimit = FORM == QOB_C128 ? 4096.f : 16384.f;
+constexpr float kSlLimit = FORM == QOB_C64 ? 2048.f : 4096.f;
 
 // A lower bound of sum |a| |x| over n indices, term (i, j): at least n less the components
 // of either side below their thresholds, 2^-(i + 1) and 2^-(j + 1), lie above both, and
@@ -331,13 +348,14 @@ __global__ void __launch_bounds__(split_threads(ROWS)) k_slice_split(const IN* _
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const C2 c = t[v * pitch + kc * 8 + 2 * p + e];
-          const long long f = fixed_point<S>(im ? c.y : c.x, ex[v]);
-          const unsigned long long mag = f < 0 ? -f : f;
+          const auto f = fixed_point<S>(im ? c.y : c.x, ex[v]);
+          const auto mag = magnitude(f);
           g[e] = digit_bytes(f);
-          levels += 1ull << (10 * min(__clzll((long long)mag) - (64 - kBits<S>), kLevels));
+          levels += 1ull << (10 * min(lead<S>(mag), kLevels));
           n1 += (uint32_t)(mag >> (kBits<S> - 14));
-          const int lo = (int)(g[e].x ^ 0x80808080u), hi = (int)((g[e].y ^ 0x80808080u) & (S == 8 ? ~0u : 0xffu));
-          n2 = __dp4a(hi, hi, __dp4a(lo, lo, n2));
+          const int lo = (int)(g[e].x ^ 0x80808080u), hi = (int)((g[e].y ^ 0x80808080u) & (S == 8 ? ~0u : 0xffffffu));
+          n2 = __dp4a(lo, lo, n2);
+          if (S > 4) n2 = __dp4a(hi, hi, n2);
         }
 #pragma unroll
         for (int s = 0; s < S; ++s) {
@@ -416,7 +434,7 @@ struct SlCfg {
   static constexpr int kSets = 2 * kCols <= 512 ? 2 : 1;     // sets in the tensor memory
   // k steps of a widened buffer (one rendezvous and its commits, ~300 cycles, beside
   // 80 or more per MMA) and of a stage
-  static constexpr int kG = S < 8 ? 2 : 1, kKs = 2;
+  static constexpr int kG = S == 4 ? 2 : 1, kKs = 2;
   static constexpr int kA = S * kSlRows * 16, kB = S * BN * 32;  // one k step: bytes of the M side, planes of the N side
   static constexpr int kWideStep = S * kSlRows * 32;             // one k step of the M side, widened
   static constexpr int kWide = kG * kWideStep;
@@ -438,7 +456,7 @@ struct SlCfg {
   static_assert(smem <= 227 * 1024, "shared memory of a block");
 };
 
-// H 2^32 + L (S = 8) or H (S = 5): the sum of the diagonals in units of the last one's
+// H 2^(8 (S - 4)) + L: the sum of the diagonals in units of the last one's
 struct Sum2 {
   long long h, l;
 };
@@ -449,12 +467,13 @@ __device__ __forceinline__ Sum2 add_diagonals(const uint32_t (&d)[S]) {
   r.h = in(0) * (1 << 24) + in(1) * (1 << 16) + in(2) * (1 << 8) + in(3);
   r.l = 0;
   if constexpr (S == 8) r.l = in(4) * (1 << 24) + in(5) * (1 << 16) + in(6) * (1 << 8) + in(7);
-  if constexpr (S == 5) r.h = r.h * (1 << 8) + in(4);  // at most 2^55: one part
+  if constexpr (S == 7) r.l = in(4) * (1 << 16) + in(5) * (1 << 8) + in(6);
   return r;
 }
-// the sum of S = 8 in units of 2^(e - 68), rounded to nearest, without the FP64 pipe
+// the sum in units of 2^(e - 36 - 8 (S - 4)), rounded to nearest, without the FP64 pipe
+template <int S>
 __device__ __forceinline__ double sum_to_double(Sum2 v, int e) {
-  constexpr int LB = 32;                        // bits of the low part's unit below the high one's
+  constexpr int LB = 8 * (S - 4);               // bits of the low part's unit below the high one's
   long long g = v.h + (v.l >> LB);              // floor
   unsigned long long f = (unsigned long long)v.l << (64 - LB);  // fraction, in units of 2^-64
   const bool neg = g < 0;
@@ -705,7 +724,7 @@ __global__ void __launch_bounds__(SlCfg<FORM, BN>::kThreads, 1)
     // the vectors [h KQ, (h + 1) KQ): their real columns and, BN/2 on, their imaginary ones
     const int q4 = warp & 3, half = (warp - 3 - C::kWidenWarps) >> 2;
     constexpr int KQ = BN / 2 / (C::kAddWarps / 4);
-    constexpr int CG = S == 5 ? 4 : 2;  // columns at a time
+    constexpr int CG = S == 4 ? 4 : 2;  // columns at a time
     const uint32_t lane_addr = tmem + ((uint32_t)(q4 * 32) << 16);
     const int r = q4 * 32 + lane, il = r >> 1;
     const bool even = (lane & 1) == 0;
@@ -750,13 +769,13 @@ __global__ void __launch_bounds__(SlCfg<FORM, BN>::kThreads, 1)
           // even lane: Re y = Re a Re x - Im a Im x; odd lane: Im y = Im a Re x + Re a Im x
           o.h = __shfl_xor_sync(0xffffffffu, o.h, 1);
           a.h += even ? -o.h : o.h;
-          if constexpr (S == 8) {
+          if constexpr (S > 4) {
             o.l = __shfl_xor_sync(0xffffffffu, o.l, 1);
             a.l += even ? -o.l : o.l;
-            got[c] = sum_to_double(a, er + __shfl_sync(0xffffffffu, ec, c0 + c));
+            got[c] = sum_to_double<S>(a, er + __shfl_sync(0xffffffffu, ec, c0 + c));
           } else {
             const int e = __shfl_sync(0xffffffffu, ec, c0 + c);
-            got[c] = __ll2float_rn(a.h) * __int_as_float((er - 22 + 127) << 23) * __int_as_float((e - 22 + 127) << 23);
+            got[c] = __ll2float_rn(a.h) * __int_as_float((er - 18 + 127) << 23) * __int_as_float((e - 18 + 127) << 23);
           }
         }
 #pragma unroll
