@@ -423,6 +423,8 @@ int dense_kchunks(int64_t m, int64_t n, int64_t ncols, int tc) {
 int dense_tile(int64_t ncols, bool ff) {
   return ncols >= 8 && !ff ? 8 : ncols >= 4 ? 4 : ncols >= 2 ? 2 : 1;
 }
+// vectors of one launch (grid.y)
+int64_t dense_launch_cols(bool ff) { return (int64_t)65535 * (ff ? 4 : 8); }
 
 template <typename CT, typename R>
 void dense_typed(const void* a, int64_t m, int64_t n, c128 alpha, const void* x, int64_t xes, int64_t xcs,
@@ -445,7 +447,7 @@ void dense_typed(const void* a, int64_t m, int64_t n, c128 alpha, const void* x,
     case 8: run(gated ? k_dense<CT, R, 8, true> : k_dense<CT, R, 8, false>); break;
     case 4: run(gated ? k_dense<CT, R, 4, true> : k_dense<CT, R, 4, false>); break;
     case 2: run(gated ? k_dense<CT, R, 2, true> : k_dense<CT, R, 2, false>); break;
-    default: run(k_dense<CT, R, 1, false>);  // a gate comes with two vectors and more
+    default: run(gated ? k_dense<CT, R, 1, true> : k_dense<CT, R, 1, false>);
   }
   if (part) {
     launch_kernel(gated, gated ? k_dense_reduce<CT, R, true> : k_dense_reduce<CT, R, false>,
@@ -473,7 +475,7 @@ void dense_ff(const void* a, int64_t m, int64_t n, c128 alpha, const void* x, in
   switch (tc) {
     case 4: run(gated ? k_dense_ff<4, true> : k_dense_ff<4, false>); break;
     case 2: run(gated ? k_dense_ff<2, true> : k_dense_ff<2, false>); break;
-    default: run(k_dense_ff<1, false>);
+    default: run(gated ? k_dense_ff<1, true> : k_dense_ff<1, false>);
   }
   if (part) {
     launch_kernel(gated, gated ? k_dense_reduce<double2, double, true> : k_dense_reduce<double2, double, false>,
@@ -485,7 +487,7 @@ void dense_ff(const void* a, int64_t m, int64_t n, c128 alpha, const void* x, in
 }  // namespace
 
 void reserve_dense(int precision, int64_t m, int64_t n, int64_t ncols, bool ff, Workspace& ws, int slot) {
-  ncols = std::min<int64_t>(ncols, 65535 * 8);  // a launch's
+  ncols = std::min<int64_t>(ncols, dense_launch_cols(ff));
   const int kch = dense_kchunks(m, n, ncols, dense_tile(ncols, ff));
   if (kch > 1) ws.get(slot, (size_t)kch * ncols * m * (precision == QOB_C128 ? 16 : 8));
 }
@@ -495,12 +497,13 @@ void launch_dense(int precision, const void* a, int64_t m, int64_t n, c128 alpha
                   int64_t ncols, cudaStream_t s, Workspace* ws, int slot, bool ff, bool dmma, FmaGate gate) {
   if (m == 0 || ncols == 0) return;
   const size_t esz = precision == QOB_C128 ? 16 : 8;
-  if (ncols > 65535 * 8) {  // grid.y limit: split the vectors
-    for (int64_t c0 = 0; c0 < ncols; c0 += 65535 * 8) {
+  const int64_t most = dense_launch_cols(ff);
+  if (ncols > most) {
+    for (int64_t c0 = 0; c0 < ncols; c0 += most) {
       launch_dense(precision, a, m, n, alpha, (const char*)x + c0 * xcs * esz, xes, xcs, beta,
-                   (char*)y + c0 * ycs * esz, yes, ycs, std::min<int64_t>(65535 * 8, ncols - c0), s, ws, slot,
+                   (char*)y + c0 * ycs * esz, yes, ycs, std::min<int64_t>(most, ncols - c0), s, ws, slot,
                    ff, dmma, gate);
-      gate.c0 += 65535 * 8;
+      gate.c0 += most;
     }
     return;
   }

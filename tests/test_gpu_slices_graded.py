@@ -226,3 +226,28 @@ def test_graded_kets_cost_what_the_fma_kernels_do(form, tol, unit, u):
         ms.append(best)
     # three launches that find nothing to do beside kernels of 50 us and more
     assert ms[0] < 2 * ms[1], ms
+
+
+@pytest.mark.parametrize("form,tol,unit,u", FORMS)
+def test_more_vectors_than_one_fma_launch(form, tol, unit, u):
+    """The gate of the second launch, of one vector: graded (left to it) and not."""
+    import torch
+
+    from qobgpu.mul import mul_
+
+    n, k = 300, (4 if form == "ff" else 8) * 65535 + 1
+    a = _rounded(_matrix(Q.Rng(8), n, n), form)
+    dt = torch.complex64 if form == "c64" else torch.complex128
+    g = torch.Generator(device="cuda:0")
+    g.manual_seed(9)
+    x = torch.randn(k, n, dtype=torch.complex64, device="cuda:0", generator=g).to(dt)
+    y0 = torch.randn(k, n, dtype=torch.complex64, device="cuda:0", generator=g).to(dt)
+    b, bk, op = Q.GenericBasis(n), Q.GenericBasis(k), _dense(a)
+    for graded in (False, True):
+        if graded:
+            x[-1, 10:] *= 2.0 ** -30
+        y = y0.clone()
+        mul_(O.Operator(b, bk, y.t()), op, O.Operator(b, bk, x.t()), 0.7, 0.3, arith="ff" if form == "ff" else None)
+        for c in (0, 40000, k - 40, k - 2, k - 1):
+            want = 0.7 * (a @ x[c].cpu().numpy().astype(np.complex128)) + 0.3 * y0[c].cpu().numpy().astype(np.complex128)
+            assert rel_l2(y[c].cpu().numpy().astype(np.complex128), want) < tol, (graded, c)
