@@ -89,12 +89,15 @@ c128 coefval(const TermCoef& c, const OpNode* root) {
 
 // Whether an m x n dense matrix on ncols columns runs from its digit planes
 // (k_slice.cu, form QOB_C128, QOB_C64 or QOB_C128X) rather than on the FMA kernels.
-// Measured, FMA -> planes, us.  Dense operators, ComplexF64: n = 4096 on 4 / 16 kets
-// 452 -> 111 / 1737 -> 115, 300 on 16 97 -> 33; double-float 170 -> 104 / 656 -> 109,
-// 61 -> 32; ComplexF32: 4096 on 4 / 8 / 16 61 -> 63 / 90 -> 64 / 157 -> 65, 300 on 16
-// 30 -> 22, 512 on 64 28 -> 28.  Mode products (two): ComplexF64 64 x 2 x 70 on 4 / 16 kets 43 -> 58
-// / 147 -> 58; double-float 64 x 2 x 70 on 16 55 -> 55, 199 x 3 x 201 on 1 143 -> 88;
-// ComplexF32 199 x 3 x 201 on 1 / 15 50 -> 52 / 474 -> 160.
+// Measured on Gaussian entries, FMA -> planes, us of a call.  Dense operators, ComplexF64: n = 4096
+// on 4 / 16 kets 457 -> 113 / 1743 -> 118, 300 on 16 101 -> 30; double-float 4096 on 2 / 4 / 16
+// 106 -> 105 / 180 -> 106 / 672 -> 111, 300 on 16 68 -> 30; ComplexF32 4096 on 8 / 16 94 -> 70 /
+// 161 -> 70 (on 4 61 -> 63 of device time: not taken), 300 on 16 35 -> 23, 512 on 64 31 -> 33.  Mode
+// products (two): ComplexF64 64 x 2 x 70 on 16 kets 152 -> 64, 40 x 5 x 48 on 16 103 -> 76;
+// double-float 64 x 2 x 70 on 16 65 -> 62, 40 x 5 x 48 on 64 133 -> 137, 199 x 3 x 201 on 1 158 -> 94;
+// ComplexF32 101 x 3 x 144 on 9 83 -> 64, 199 x 3 x 201 on 2 / 15 95 -> 64 / 475 -> 175.  Kets that
+// the planes leave to the FMA kernels pay for the split: dense 4096 on 16 kets, ComplexF64 1743 ->
+// 1757, double-float 671 -> 672, ComplexF32 161 -> 170.
 bool slices_pay(int form, int64_t m, int64_t n, int64_t ncols, bool mode) {
   if (m < kSliceMin || n < kSliceMin || ncols < 2 || ncols >= (int64_t(1) << 30)) return false;
   const double flops = 8.0 * m * n * ncols;

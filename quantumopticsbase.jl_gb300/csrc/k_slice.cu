@@ -56,10 +56,10 @@
 // over one block per SM; a run's part of a row tile either covers it (written to y)
 // or goes to a partial product that k_slice_reduce adds in chunk order.  Waits are
 // bounded as in k_tc32.cu.
-// Measured (device time of a call, FMA kernels -> this; one GB300): two mode products
-// with 199 x 199 and 201 x 201 factors on 15 kets, ComplexF64 4786 -> 341 us,
-// double-float 1331 -> 316, ComplexF32 474 -> 160; a 4096 x 4096 operator on 16 kets
-// 1737 -> 115, 656 -> 109, 157 -> 65.  Error against 128-bit products: ComplexF64
+// Measured (a call among others, Gaussian entries, FMA kernels -> this; one GB300): two mode products
+// with 199 x 199 and 201 x 201 factors on 15 kets, ComplexF64 4791 -> 343 us,
+// double-float 1412 -> 322, ComplexF32 475 -> 175; a 4096 x 4096 operator on 16 kets
+// 1743 -> 118, 672 -> 111, 161 -> 70.  Error against 128-bit products: ComplexF64
 // 1e-16 (FMA 4e-16), double-float 1e-15 (4e-14), ComplexF32 6e-8 (2e-7).  Bound by
 // the tensor pipe's rate on short MMAs (80 to 110 cycles each up to N = 160) with
 // their commits and, on many columns, by adding up the diagonals (about 9000 cycles
