@@ -122,8 +122,10 @@ void apply_plan(Context& ctx, Plan& P, c128 alpha, const void* x, int64_t xes, i
   const size_t esz = P.precision == QOB_C128 ? 16 : 8;
   const c128 one{1.0, 0.0}, zero{0.0, 0.0};
   if (P.kind == Plan::Kind::Sum) {
-    // LazySum with no terms or alpha == 0: _zero_op_mul! (src/operators_lazysum.jl:190-192)
-    if (is_zero(alpha) || P.nterms_total == 0) {
+    // LazySum with no terms or alpha == 0: _zero_op_mul! (src/operators_lazysum.jl:190-192), and
+    // terms without a single stored entry
+    const bool empty = !P.gather && P.dense.empty() && P.modek.empty() && P.subs.empty();
+    if (is_zero(alpha) || P.nterms_total == 0 || empty) {
       launch_scale(P.precision, y, P.m, ncols, yes, ycs, beta, s);
       return;
     }
