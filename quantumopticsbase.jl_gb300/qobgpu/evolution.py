@@ -11,6 +11,7 @@
 from __future__ import annotations
 
 import ctypes as C
+import weakref
 
 import numpy as np
 
@@ -39,6 +40,8 @@ class Batch:
         p = C.c_void_p()
         raise_for(L.lib().qob_batch_create(self.ctx.ptr, code, C.byref(p)), self.ctx)
         self.ptr = p
+        # at exit finalizers run newest first: the batch goes before its context
+        self._finalizer = weakref.finalize(self, L.lib().qob_batch_free, self.ctx.ptr, p)
         self._keep = []
 
     def add(self, op, x, y, alpha=1.0, beta=0.0):
@@ -66,13 +69,6 @@ class Batch:
         v = (C.c_int64 * 5)()
         raise_for(L.lib().qob_batch_info(self.ctx.ptr, self.ptr, v), self.ctx)
         return {"items": v[0], "fused": v[1], "tiles": v[2], "tile": v[3], "grid": v[4]}
-
-    def __del__(self):
-        try:
-            if self.ptr:
-                L.lib().qob_batch_free(self.ctx.ptr, self.ptr)
-        except Exception:
-            pass
 
 
 def factor_rows(H: O.TimeDependentSum, t0: float, dt: float, nsteps: int) -> np.ndarray:
