@@ -4,6 +4,7 @@
 #include <atomic>
 #include <cstring>
 #include <new>
+#include <optional>
 
 #include "fft_line.h"
 #include "qob_internal.h"
@@ -78,6 +79,7 @@ Context::~Context() {
     if (e) cudaEventDestroy(e);
   for (auto e : ticket_done)
     if (e) cudaEventDestroy(e);
+  if (slice_done) cudaEventDestroy(slice_done);
 }
 
 namespace {
@@ -105,6 +107,35 @@ bool slices_pay(int form, int64_t m, int64_t n, int64_t ncols, bool mode) {
   if (form == QOB_C64) return ncols >= 8 && flops >= 1e7;
   return flops >= (ncols >= 4 ? 1e7 : 1e8);
 }
+
+// One product from digit planes: it starts after the context's last one, if that was on another
+// stream, since both use the same workspace, which is theirs alone.  The FMA kernels use none on
+// many vectors, so that such calls may come from several streams.  The launch of a recorded
+// product (qob_graph_launch) takes its turn too.
+struct SliceTurn {
+  Context& ctx;
+  cudaStream_t s;
+  bool eager;
+  SliceTurn(Context& c, cudaStream_t stream) : ctx(c), s(stream) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    QOB_CUDA(cudaStreamIsCapturing(s, &cs));
+    eager = cs == cudaStreamCaptureStatusNone;
+    if (!eager) {
+      ctx.slice_recorded = true;
+      return;
+    }
+    unsigned long long id = 0;
+    QOB_CUDA(cudaStreamGetId(s, &id));
+    if (!ctx.slice_done)
+      QOB_CUDA(cudaEventCreateWithFlags(&ctx.slice_done, cudaEventDisableTiming));
+    else if (id != ctx.slice_stream)
+      QOB_CUDA(cudaStreamWaitEvent(s, ctx.slice_done, 0));
+    ctx.slice_stream = id;
+  }
+  void end() {  // behind the last launch that reads the workspace
+    if (eager) QOB_CUDA(cudaEventRecord(ctx.slice_done, s));
+  }
+};
 
 int64_t prod_range(const std::vector<int64_t>& v, size_t lo, size_t hi) {
   int64_t p = 1;
@@ -152,20 +183,22 @@ void apply_plan(Context& ctx, Plan& P, c128 alpha, const void* x, int64_t xes, i
     }
     for (auto& d : P.dense) {
       // partial sums of a split product in slot ws (free here, as for the split input above);
-      // a double-float plan splits x into slot ws + 1 first; digit planes use ws + 2 and
-      // ws + 3 (sub-plans run after), and the tiles they leave go to the FMA kernels
+      // a double-float plan splits x into slot ws + 1 first; the tiles that digit planes
+      // leave go to the FMA kernels
       const c128 ad = cmul(alpha, coefval(d.coef, P.root));
       const int form = P.ff ? QOB_C128X : P.precision;
       TcColMap xm, ym;
       xm.st = xcs;
       ym.st = ycs;
       FmaGate gate;
+      std::optional<SliceTurn> turn;
       const void* xin = x;
       void* xs = P.ff ? ctx.ws.get(ws + 1, (size_t)((P.n - 1) * xes + (ncols - 1) * xcs + 1) * 16) : nullptr;
       if (!(form == QOB_C64 ? ctx.fp32_tensor : ctx.fp64_tensor && !P.ff) && slices_pay(form, d.m, d.n, ncols, false) &&
           slice_ready(d.sl, form, d.a.p, d.m, d.n, slice_swap(yes, ym, ncols), s)) {
+        turn.emplace(ctx, s);
         reserve_dense(P.precision, d.m, d.n, ncols, P.ff, ctx.ws, ws);  // before the planes take what is free
-        gate = launch_slices(d.sl, form, ad, x, xes, xm, b, y, yes, ym, ncols, s, &ctx.ws, ws + 2,
+        gate = launch_slices(d.sl, form, ad, x, xes, xm, b, y, yes, ym, ncols, s, &ctx.slice_ws,
                              static_cast<unsigned*>(ctx.status.p), ctx.num_sms, ctx.pdl);
       }
       if (P.ff) {
@@ -180,6 +213,7 @@ void apply_plan(Context& ctx, Plan& P, c128 alpha, const void* x, int64_t xes, i
         launch_dense(P.precision, d.a.p, d.m, d.n, ad, xin, xes, xcs, b, y, yes, ycs, ncols, s, &ctx.ws, ws, P.ff,
                      ctx.fp64_tensor, gate);
       }
+      if (turn) turn->end();
       b = one;
     }
     for (auto& mk : P.modek) {
@@ -229,9 +263,12 @@ void apply_plan(Context& ctx, Plan& P, c128 alpha, const void* x, int64_t xes, i
           const void* sin = src;
           const int64_t len_in = prod_range(cur, 0, cur.size());
           void* xs = ffs ? ctx.ws.get(ws + 2, (size_t)((len_in - 1) * ses + (ncols - 1) * scs + 1) * 16) : nullptr;
-          if (slices)
-            gate = launch_slices(st.sl, form, ak, src, s1 * ses, xm, bk, out, s1 * out_es, ym, pcols, s, &ctx.ws, ws + 3,
-                                 status, ctx.num_sms, ctx.pdl);
+          std::optional<SliceTurn> turn;
+          if (slices) {
+            turn.emplace(ctx, s);
+            gate = launch_slices(st.sl, form, ak, src, s1 * ses, xm, bk, out, s1 * out_es, ym, pcols, s,
+                                 &ctx.slice_ws, status, ctx.num_sms, ctx.pdl);
+          }
           if (ffs) {
             launch_ff_split(src, len_in, ncols, ses, scs, xs, s, gate.any);
             sin = xs;
@@ -244,6 +281,7 @@ void apply_plan(Context& ctx, Plan& P, c128 alpha, const void* x, int64_t xes, i
             launch_modek(P.precision, st.a.p, st.eye, s1, st.dout, st.din, s3, ak, sin, ses, scs, bk, out, out_es,
                          out_cs, ncols, s, ffs, ctx.fp64_tensor, gate);
           }
+          if (turn) turn->end();
         };
         if (last) {
           mode_product(b, y);
@@ -853,7 +891,7 @@ int qob_op_set_tile(qob_ctx* ctx, qob_op* op, int side, int dtype, int vectors_p
 // without memory (0: no limit).
 int qob_debug_limit_workspace(qob_ctx* ctx, size_t bytes) {
   if (!ctx) return QOB_ERR_ARG;
-  ctx->c.ws.limit = bytes ? bytes : SIZE_MAX;
+  ctx->c.ws.limit = ctx->c.slice_ws.limit = bytes ? bytes : SIZE_MAX;
   return QOB_OK;
 }
 
@@ -1116,12 +1154,14 @@ int qob_dot(qob_ctx* ctx, int dtype, const void* x, const void* y, int64_t n, do
 struct qob_graph {
   cudaGraph_t g = nullptr;
   cudaGraphExec_t e = nullptr;
+  bool slices = false;  // holds a product from digit planes
 };
 
 int qob_graph_begin(qob_ctx* ctx, void* stream) {
   return guard(ctx, [&] {
     if (!ctx || !stream) fail(QOB_ERR_ARG, "capture needs a context and a non-default stream");
     QOB_CUDA(cudaStreamBeginCapture((cudaStream_t)stream, cudaStreamCaptureModeThreadLocal));
+    ctx->c.slice_recorded = false;
   });
 }
 
@@ -1129,6 +1169,7 @@ int qob_graph_end(qob_ctx* ctx, void* stream, qob_graph** out) {
   return guard(ctx, [&] {
     if (!ctx || !stream || !out) fail(QOB_ERR_ARG, "qob_graph_end: bad arguments");
     auto* gr = new qob_graph;
+    gr->slices = ctx->c.slice_recorded;
     cudaError_t e = cudaStreamEndCapture((cudaStream_t)stream, &gr->g);
     if (e != cudaSuccess) {
       delete gr;
@@ -1147,7 +1188,10 @@ int qob_graph_end(qob_ctx* ctx, void* stream, qob_graph** out) {
 int qob_graph_launch(qob_ctx* ctx, qob_graph* graph, void* stream) {
   return guard(ctx, [&] {
     if (!graph) fail(QOB_ERR_ARG, "null graph");
+    std::optional<SliceTurn> turn;
+    if (graph->slices) turn.emplace(ctx->c, (cudaStream_t)stream);
     QOB_CUDA(cudaGraphLaunch(graph->e, (cudaStream_t)stream));
+    if (turn) turn->end();
   });
 }
 

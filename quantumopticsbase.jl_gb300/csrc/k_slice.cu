@@ -914,7 +914,7 @@ void run_split(const IN* x, int64_t n, int64_t es, const TcColMap& map, int64_t 
 // swap: the vectors are the M side (their bytes widened), the matrix the N side.
 template <int FORM, int BN>
 FmaGate run_slices(const SliceDense& d, bool swap, const void* xv, int64_t xes, const TcColMap& xm, int64_t ncols, void* yv,
-                   int64_t yes, const TcColMap& ym, c128 al, c128 be, Workspace* ws, int slot, cudaStream_t s,
+                   int64_t yes, const TcColMap& ym, c128 al, c128 be, Workspace* ws, cudaStream_t s,
                    unsigned* status, int num_sms, bool pdl) {
   using C = SlCfg<FORM, BN>;
   using V = typename Sl<FORM>::V;
@@ -940,14 +940,14 @@ FmaGate run_slices(const SliceDense& d, bool swap, const void* xv, int64_t xes, 
   const SlicePlanes& pl = swap ? d.nside : d.mside;
   const SliceSide* sides = static_cast<const SliceSide*>(pl.sides);
   const size_t bbytes = (size_t)vt * nkb * (swap ? C::kA : C::kB), ebytes = ((size_t)vt * (nch * (tile + 1) + 1) + 1) * sizeof(int);
-  unsigned char* w = static_cast<unsigned char*>(ws->try_get(slot, bbytes + ebytes, s));
+  unsigned char* w = static_cast<unsigned char*>(ws->try_get(0, bbytes + ebytes, s));
   if (!w) return FmaGate();
   int* exps = reinterpret_cast<int*>(w + bbytes);
   int* flags = exps + vt * nch * tile;
   int *left = flags + vt * nch, *any = left + vt;
   V* part = nullptr;
   if (per % nch != 0) {
-    part = static_cast<V*>(ws->try_get(slot + 1, (size_t)rtiles * smax * H * HM * sizeof(V), s));
+    part = static_cast<V*>(ws->try_get(1, (size_t)rtiles * smax * H * HM * sizeof(V), s));
     if (!part) return FmaGate();
   }
   if (swap)
@@ -1077,10 +1077,10 @@ bool slice_ready(SliceDense& d, int form, const void* a, int64_t m, int64_t n, b
 
 FmaGate launch_slices(const SliceDense& d, int form, c128 alpha, const void* x, int64_t xes, const TcColMap& xm,
                       c128 beta, void* y, int64_t yes, const TcColMap& ym, int64_t ncols, cudaStream_t s, Workspace* ws,
-                      int slot, unsigned* status, int num_sms, bool pdl) {
+                      unsigned* status, int num_sms, bool pdl) {
   const bool swap = slice_swap(yes, ym, ncols);
 #define QOB_SL(F, BN) \
-  run_slices<F, BN>(d, swap, x, xes, xm, ncols, y, yes, ym, alpha, beta, ws, slot, s, status, num_sms, pdl)
+  run_slices<F, BN>(d, swap, x, xes, xm, ncols, y, yes, ym, alpha, beta, ws, s, status, num_sms, pdl)
   if (form == QOB_C128) return ncols <= 16 ? QOB_SL(QOB_C128, 32) : QOB_SL(QOB_C128, kSwapBN);
   if (form == QOB_C128X) return ncols <= 16 ? QOB_SL(QOB_C128X, 32) : QOB_SL(QOB_C128X, kSwapBN);
   return ncols <= 16 ? QOB_SL(QOB_C64, 32) : QOB_SL(QOB_C64, kSwapBN);

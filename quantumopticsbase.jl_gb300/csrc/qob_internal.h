@@ -461,6 +461,12 @@ struct Context {
   // bounded waits that gave up and failed debug checks; read by qob_device_status
   DeviceBuf status;
   DeviceBuf grid_bar;  // the grid barrier's counter (rk4.cu)
+  // the workspace of products from digit planes, one at a time: the end of the last one and
+  // the id of its stream (SliceTurn, capi.cu)
+  Workspace slice_ws;
+  cudaEvent_t slice_done = nullptr;
+  unsigned long long slice_stream = 0;
+  bool slice_recorded = false;  // one was recorded in a capture since qob_graph_begin
   ~Context();
 };
 
@@ -537,7 +543,7 @@ bool launch_gemm_tc(const TcDense& d, c128 alpha, const void* x, int64_t xes, co
 // QOB_C64 or QOB_C128X) from its digit planes (k_slice.cu): columns as
 // launch_gemm_tc's; x unsplit.  slice_swap: which side the vectors take; slice_ready
 // makes the matrix's planes for it if they are not there yet (not inside a capture)
-// and says whether they can be used.  Workspace slots slot, slot + 1.  The columns of
+// and says whether they can be used.  Workspace slots 0 and 1, of one product at a time.  The columns of
 // the tiles that the returned gate names are not written: the FMA kernels follow with it.
 // Without room for the vectors' planes nothing is done and the gate is open to every column.
 constexpr int64_t kSliceMin = 32;  // rows and columns from which a matrix gets planes
@@ -545,7 +551,7 @@ bool slice_swap(int64_t yes, const TcColMap& ym, int64_t ncols);
 bool slice_ready(SliceDense& d, int form, const void* a, int64_t m, int64_t n, bool swap, cudaStream_t s);
 FmaGate launch_slices(const SliceDense& d, int form, c128 alpha, const void* x, int64_t xes, const TcColMap& xm,
                       c128 beta, void* y, int64_t yes, const TcColMap& ym, int64_t ncols, cudaStream_t s, Workspace* ws,
-                      int slot, unsigned* status, int num_sms, bool pdl);
+                      unsigned* status, int num_sms, bool pdl);
 // contracted dimension and kets from which the FP64 tensor-core option
 // applies (an 8 x 8 x 4 tile covers 8 kets: on one ket the FMA kernels are
 // about 15x faster at n = 4096)
