@@ -49,6 +49,7 @@ void* Workspace::get(size_t slot, size_t bytes) {
 #endif
     // buffers are reused across calls; wait for work that may still use the old one
     QOB_CUDA(cudaDeviceSynchronize());
+    if (recorded && d.p) kept.push_back(std::move(d));
     d.alloc(bytes + bytes / 4);
   }
   return d.p;
@@ -122,6 +123,7 @@ struct SliceTurn {
     eager = cs == cudaStreamCaptureStatusNone;
     if (!eager) {
       ctx.slice_recorded = true;
+      ctx.ws.recorded = ctx.slice_ws.recorded = true;
       return;
     }
     unsigned long long id = 0;
@@ -1162,6 +1164,7 @@ int qob_graph_begin(qob_ctx* ctx, void* stream) {
     if (!ctx || !stream) fail(QOB_ERR_ARG, "capture needs a context and a non-default stream");
     QOB_CUDA(cudaStreamBeginCapture((cudaStream_t)stream, cudaStreamCaptureModeThreadLocal));
     ctx->c.slice_recorded = false;
+    ctx->c.ws.recorded = true;
   });
 }
 

@@ -419,6 +419,10 @@ struct Plan {
 // ---------------------------------------------------------------------------
 struct Workspace {
   std::vector<DeviceBuf> slots;
+  // set once a capture has seen the buffers: one that has to grow is then kept until the
+  // context ends, since a graph still uses it (each is 1.25 times the one before, or more)
+  bool recorded = false;
+  std::vector<DeviceBuf> kept;
   void* get(size_t slot, size_t bytes);
   // the same for work that has another way: null where there is no memory for it, or the
   // slot would grow while s is captured
