@@ -534,7 +534,8 @@ int qob_server_destroy(qob_server* server);
  * qob_* calls issued on `stream` (a non-default stream) are recorded instead of
  * run; qob_graph_launch replays them.  Operators used inside must have been
  * applied (or qob_op_prepare'd) once with the same shapes before capture, so
- * that no allocation or upload happens while recording.
+ * that no allocation or upload happens while recording.  Replays use the context's
+ * workspace as the recorded calls did, which is kept for them.
  * ------------------------------------------------------------------------- */
 typedef struct qob_graph qob_graph;
 int qob_graph_begin(qob_ctx* ctx, void* stream);
